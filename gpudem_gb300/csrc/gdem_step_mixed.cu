@@ -1392,15 +1392,6 @@ int kernel_kind(const View<Mixed>& v) {
     }();
     return k;
 }
-int sm_count() {
-    static const int c = [] {
-        int dev = 0, cnt = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&cnt, cudaDevAttrMultiProcessorCount, dev);
-        return cnt > 0 ? cnt : 1;
-    }();
-    return c;
-}
 }  // namespace
 
 StepLaunch step_launch(const View<Mixed>& v, int reserve) {
