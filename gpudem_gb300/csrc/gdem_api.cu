@@ -7,6 +7,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -26,6 +28,14 @@
 namespace gdem {
 template <class T>
 void launch_gather_positions(const View<T>& v, double* out, cudaStream_t st);
+template <class T>
+void launch_gather_state(const View<T>& v, double* out, int* active, cudaStream_t st);
+template <class T>
+void launch_gather_forces(const View<T>& v, double* out, cudaStream_t st);
+template <class T>
+void launch_gather_counts(const View<T>& v, int wall, int* out, cudaStream_t st);
+template <class T>
+void launch_gather_history(const View<T>& v, int wall, int rows, cudaStream_t st);
 }
 
 using namespace gdem;
@@ -225,7 +235,8 @@ struct Impl : EngineBase {
     char* cell_arena = nullptr;
     double* stats_partials = nullptr;
     int stats_nblk = 0;
-    double* gather = nullptr;  // [3n] pId-ordered positions for fast exports
+    double* gather = nullptr;  // [13n] pId-ordered state for exports (x, v, angv, r, m, k, etaconst) ...
+    int* gather_i = nullptr;   // ... and [n] activity or history lengths
     cudaGraphExec_t gK = nullptr, g1 = nullptr;
     int K = 8;
     bool use_graphs = true;
@@ -340,7 +351,8 @@ struct Impl : EngineBase {
         A.add(&v.ctl, 1);
         stats_nblk = stats_blocks(n);
         A.add(&stats_partials, (size_t)16 * stats_nblk);
-        A.add(&gather, (size_t)3 * n);
+        A.add(&gather, (size_t)13 * n);
+        A.add(&gather_i, n);
         CKE(cudaMalloc((void**)&arena, A.total()));
         A.bind(arena);
         CKE(cudaMemsetAsync(arena, 0, A.total(), st));
@@ -854,99 +866,98 @@ struct Impl : EngineBase {
         return GDEM_OK;
     }
 
+    // Every page of [p, p + bytes) mapped for writing, its contents kept: an
+    // output array fresh from the allocator otherwise takes its page faults
+    // inside the copy (4.0 ms instead of 0.6 for 104 MB).  Called before the wait
+    // for the stream, so it runs while queued steps do.  Where the system cannot
+    // do it, the copy faults them in as before.
+    static void map_pages(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+        const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+        if (!p || bytes < 4 * page) return;
+        const size_t a = reinterpret_cast<size_t>(p) & ~(page - 1), e = reinterpret_cast<size_t>(p) + bytes;
+        madvise(reinterpret_cast<void*>(a), (e - a + page - 1) & ~(page - 1), MADV_POPULATE_WRITE);
+#else
+        (void)p;
+        (void)bytes;
+#endif
+    }
+
+    // The state is gathered into pId order on the device and copied straight
+    // into the caller's arrays (a million spheres: 61 ms when the arrays came
+    // in storage order and the host permuted them, 4.1 ms now, of which 1 ms
+    // is left when steps are queued before it).
     int export_(gdem_particles* p) override {
-        Ctl c;
-        std::vector<int> pid;
-        int rc = current(c, pid);
-        if (rc) return rc;
-        const SBank<T>& S = v.S[c.s];
-        const PBank<T>& P = v.P[c.p];
-        std::vector<double4_32a> pos;
-        std::vector<V4> vel, rot, mat;
-        if ((rc = dl(vel, S.vel, n)) || (rc = dl(rot, S.rot, n)) || (rc = dl(mat, P.mat, n))) return rc;
-        if (T::mixed) {
-            std::vector<float4> ph, pl;
-            if ((rc = dl(ph, S.posh, n)) || (rc = dl(pl, S.posl, n))) return rc;
-            pos.resize(n);
-            for (int i = 0; i < n; i++)
-                pos[i] = make_double4_32a((double)ph[i].x + (double)pl[i].x, (double)ph[i].y + (double)pl[i].y,
-                                          (double)ph[i].z + (double)pl[i].z,
-                                          (double)fabsf(ph[i].w) + (double)pl[i].w);
-        } else if ((rc = dl(pos, S.pos, n))) {
-            return rc;
-        }
-        std::vector<float4> vl, wl;
-        if (T::mixed && ((rc = dl(vl, S.vell, n)) || (rc = dl(wl, S.rotl, n)))) return rc;
-        auto lo = [&](const std::vector<float4>& a, int i, int c) -> double {
-            if (!T::mixed) return 0.;
-            return c == 0 ? a[i].x : (c == 1 ? a[i].y : a[i].z);
+        struct Field {
+            void* dst;
+            const void* src;
+            size_t bytes;
         };
-        for (int i = 0; i < n; i++) {
-            const int q = pid[i];
-            if (p->x) { p->x[3 * q] = pos[i].x; p->x[3 * q + 1] = pos[i].y; p->x[3 * q + 2] = pos[i].z; }
-            if (p->v) {
-                p->v[3 * q] = (double)vel[i].x + lo(vl, i, 0);
-                p->v[3 * q + 1] = (double)vel[i].y + lo(vl, i, 1);
-                p->v[3 * q + 2] = (double)vel[i].z + lo(vl, i, 2);
-            }
-            if (p->angv) {
-                p->angv[3 * q] = (double)rot[i].x + lo(wl, i, 0);
-                p->angv[3 * q + 1] = (double)rot[i].y + lo(wl, i, 1);
-                p->angv[3 * q + 2] = (double)rot[i].z + lo(wl, i, 2);
-            }
-            if (p->isActive) p->isActive[q] = rot[i].w == R(1) ? 1 : 0;
-            if (p->r) p->r[q] = pos[i].w;
-            if (p->m) p->m[q] = 1. / (double)vel[i].w;
-            if (p->k) p->k[q] = mat[i].x;
-            if (p->etaconst) p->etaconst[q] = mat[i].y;
-        }
+        const size_t N = n, D = sizeof(double);
+        const Field f[8] = {{p->x, gather, 3 * N * D},          {p->v, gather + 3 * N, 3 * N * D},
+                            {p->angv, gather + 6 * N, 3 * N * D}, {p->r, gather + 9 * N, N * D},
+                            {p->m, gather + 10 * N, N * D},     {p->k, gather + 11 * N, N * D},
+                            {p->etaconst, gather + 12 * N, N * D}, {p->isActive, gather_i, N * sizeof(int)}};
+        launch_gather_state(v, gather, gather_i, st);
+        CKE(cudaGetLastError());
+        for (const Field& q : f) map_pages(q.dst, q.bytes);
+        for (const Field& q : f)
+            if (q.dst) CKE(cudaMemcpyAsync(q.dst, q.src, q.bytes, cudaMemcpyDeviceToHost, st));
+        CKE(cudaStreamSynchronize(st));
         if (p->f || p->mom) {
             if (!v.store_forces) return failv(err, GDEM_ERR_STATE, "forces not stored (store_forces=0)");
-            std::vector<double> a, b, cc;
-            auto vec3 = [&](double* out, const double* X, const double* Y, const double* Z) -> int {
-                int r2 = dl(a, X, n) | dl(b, Y, n) | dl(cc, Z, n);
-                if (r2) return r2;
-                for (int i = 0; i < n; i++) {
-                    out[3 * pid[i]] = a[i];
-                    out[3 * pid[i] + 1] = b[i];
-                    out[3 * pid[i] + 2] = cc[i];
-                }
-                return 0;
-            };
-            if (p->f && (rc = vec3(p->f, v.fx, v.fy, v.fz))) return rc;
-            if (p->mom && (rc = vec3(p->mom, v.tx, v.ty, v.tz))) return rc;
+            launch_gather_forces(v, gather, st);
+            CKE(cudaGetLastError());
+            if (p->f) CKE(cudaMemcpyAsync(p->f, gather, 3 * N * D, cudaMemcpyDeviceToHost, st));
+            if (p->mom) CKE(cudaMemcpyAsync(p->mom, gather + 3 * N, 3 * N * D, cudaMemcpyDeviceToHost, st));
+            CKE(cudaStreamSynchronize(st));
         }
         const int stv = p->hist_stride;
-        auto hist = [&](int* cnt, int* ind, double* X, double* Y, double* Z, const int* dn, const int* did,
-                        const R* dx, const R* dy, const R* dz, int cap) -> int {
-            std::vector<int> nc, id;
-            std::vector<R> hx, hy, hz;
-            int r2;
-            if ((r2 = dl(nc, dn, n)) || (r2 = dl(id, did, (size_t)n * cap)) || (r2 = dl(hx, dx, (size_t)n * cap)) ||
-                (r2 = dl(hy, dy, (size_t)n * cap)) || (r2 = dl(hz, dz, (size_t)n * cap)))
-                return r2;
-            for (int i = 0; i < n; i++) {
-                const int q = pid[i];
-                cnt[q] = nc[i];
-                for (int s2 = 0; s2 < nc[i] && s2 < stv; s2++) {
-                    const size_t src = (size_t)s2 * n + i, dst = (size_t)q * stv + s2;
-                    // mixed-mode particle keys are storage indices: report pIds
-                    if (ind) ind[dst] = (T::mixed && did == P.hid) ? pid[id[src]] : id[src];
-                    if (X) X[dst] = hx[src];
-                    if (Y) Y[dst] = hy[src];
-                    if (Z) Z[dst] = hz[src];
+        if (stv <= 0 || !(p->numCont || p->numContWall)) return GDEM_OK;
+        Ctl c;
+        CKE(cudaMemcpy(&c, v.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
+        const PBank<T>& O = v.P[c.p ^ 1];  // where the gathered rows land
+        // each row's live prefix into the caller's strided rows
+        auto hist = [&](int wall, int* cnt, int* ind, double* X, double* Y, double* Z, const int* did, const R* dx,
+                        const R* dy, const R* dz) -> int {
+            launch_gather_counts(v, wall, gather_i, st);
+            CKE(cudaGetLastError());
+            CKE(cudaMemcpyAsync(cnt, gather_i, N * sizeof(int), cudaMemcpyDeviceToHost, st));
+            CKE(cudaStreamSynchronize(st));
+            int rows = 0;
+            for (int q = 0; q < n; q++) rows = std::max(rows, std::min(cnt[q], stv));
+            if (rows == 0 || !(ind || X || Y || Z)) return GDEM_OK;
+            launch_gather_history(v, wall, rows, st);
+            CKE(cudaGetLastError());
+            const size_t total = N * rows;
+            HostBuf<int> id(ind ? total : 0);
+            HostBuf<R> hx(X ? total : 0), hy(Y ? total : 0), hz(Z ? total : 0);
+            if (ind) CKE(cudaMemcpyAsync(id.data(), did, total * sizeof(int), cudaMemcpyDeviceToHost, st));
+            if (X) CKE(cudaMemcpyAsync(hx.data(), dx, total * sizeof(R), cudaMemcpyDeviceToHost, st));
+            if (Y) CKE(cudaMemcpyAsync(hy.data(), dy, total * sizeof(R), cudaMemcpyDeviceToHost, st));
+            if (Z) CKE(cudaMemcpyAsync(hz.data(), dz, total * sizeof(R), cudaMemcpyDeviceToHost, st));
+            CKE(cudaStreamSynchronize(st));
+            host_parallel_for(n, [&](int lo, int hi) {
+                for (int q = lo; q < hi; q++) {
+                    const size_t src = (size_t)q * rows, dst = (size_t)q * stv;
+                    const int live = std::min(cnt[q], stv);
+                    for (int k = 0; k < live; k++) {
+                        if (ind) ind[dst + k] = id[src + k];
+                        if (X) X[dst + k] = hx[src + k];
+                        if (Y) Y[dst + k] = hy[src + k];
+                        if (Z) Z[dst + k] = hz[src + k];
+                    }
                 }
-            }
-            return 0;
+            });
+            return GDEM_OK;
         };
-        if (p->numCont && stv > 0 &&
-            (rc = hist(p->numCont, p->indHis, p->deltHisx, p->deltHisy, p->deltHisz, P.nc, P.hid, P.hx, P.hy,
-                       P.hz, v.hist_cap)))
-            return rc;
-        if (p->numContWall && stv > 0 &&
-            (rc = hist(p->numContWall, p->indHisWall, p->deltHisxWall, p->deltHisyWall, p->deltHiszWall, P.ncw,
-                       P.hwid, P.hwx, P.hwy, P.hwz, v.histw_cap)))
-            return rc;
+        if (p->numCont)
+            if (int rc = hist(0, p->numCont, p->indHis, p->deltHisx, p->deltHisy, p->deltHisz, O.hid, O.hx, O.hy, O.hz))
+                return rc;
+        if (p->numContWall)
+            if (int rc = hist(1, p->numContWall, p->indHisWall, p->deltHisxWall, p->deltHisyWall, p->deltHiszWall,
+                              O.hwid, O.hwx, O.hwy, O.hwz))
+                return rc;
         return GDEM_OK;
     }
 

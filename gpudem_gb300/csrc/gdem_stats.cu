@@ -127,6 +127,108 @@ void launch_gather_positions(const View<T>& v, double* out, cudaStream_t st) {
     k_gather_positions<T><<<(v.n + kBlock - 1) / kBlock, kBlock, 0, st>>>(v, out);
 }
 
+// The whole state in pId order, the reference layout of copyFromDevice: out
+// holds x, v, angv [3n each], r, m, k, etaconst [n each], active [n].  A copy
+// bound by the scattered 8-byte writes (pIds are unrelated to storage order).
+template <class T>
+__global__ void k_gather_state(View<T> v, double* out, int* active) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= v.n) return;
+    const size_t n = v.n;
+    const SBank<T> S = v.S[v.ctl->s];
+    const PBank<T> P = v.P[v.ctl->p];
+    const double4_32a p = load_pos(S, i);
+    const typename T::v4 vel = S.vel[i], rot = S.rot[i], mat = P.mat[i];
+    const size_t q = P.pid[i];
+    double l[6] = {0., 0., 0., 0., 0., 0.};
+    if constexpr (T::mixed) {
+        const float4 vl = S.vell[i], wl = S.rotl[i];
+        l[0] = vl.x; l[1] = vl.y; l[2] = vl.z;
+        l[3] = wl.x; l[4] = wl.y; l[5] = wl.z;
+    }
+    double *x = out + 3 * q, *u = out + 3 * (n + q), *w = out + 3 * (2 * n + q), *c = out + 9 * n + q;
+    x[0] = p.x; x[1] = p.y; x[2] = p.z;
+    u[0] = (double)vel.x + l[0]; u[1] = (double)vel.y + l[1]; u[2] = (double)vel.z + l[2];
+    w[0] = (double)rot.x + l[3]; w[1] = (double)rot.y + l[4]; w[2] = (double)rot.z + l[5];
+    c[0] = p.w;
+    c[n] = 1. / (double)vel.w;
+    c[2 * n] = mat.x;
+    c[3 * n] = mat.y;
+    active[q] = rot.w == 1 ? 1 : 0;
+}
+
+// The last step's forces and torques in pId order: f, mom [3n each].
+template <class T>
+__global__ void k_gather_forces(View<T> v, double* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= v.n) return;
+    const size_t n = v.n, q = v.P[v.ctl->p].pid[i];
+    double *f = out + 3 * q, *m = out + 3 * (n + q);
+    f[0] = v.fx[i]; f[1] = v.fy[i]; f[2] = v.fz[i];
+    m[0] = v.tx[i]; m[1] = v.ty[i]; m[2] = v.tz[i];
+}
+
+// History lengths in pId order, particle (wall = 0) or wall contacts.
+template <class T>
+__global__ void k_gather_counts(View<T> v, int wall, int* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= v.n) return;
+    const PBank<T> P = v.P[v.ctl->p];
+    out[P.pid[i]] = wall ? P.ncw[i] : P.nc[i];
+}
+
+// The first `rows` history slots of every particle in pId order, row by row
+// ([n * rows]): keys (partners as pIds) and springs, into the property bank
+// that holds nothing between list rebuilds.
+template <class T>
+__global__ void k_gather_history(View<T> v, int wall, int rows) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= v.n) return;
+    const PBank<T> P = v.P[v.ctl->p], O = v.P[v.ctl->p ^ 1];
+    const int cnt = min(wall ? P.ncw[i] : P.nc[i], rows);
+    const size_t at = (size_t)P.pid[i] * rows;
+    for (int s = 0; s < cnt; s++) {
+        const size_t h = (size_t)s * v.n + i;
+        if (wall) {
+            O.hwid[at + s] = P.hwid[h];
+            O.hwx[at + s] = P.hwx[h];
+            O.hwy[at + s] = P.hwy[h];
+            O.hwz[at + s] = P.hwz[h];
+        } else {
+            // mixed-mode keys are storage indices
+            O.hid[at + s] = T::mixed ? P.pid[P.hid[h]] : P.hid[h];
+            O.hx[at + s] = P.hx[h];
+            O.hy[at + s] = P.hy[h];
+            O.hz[at + s] = P.hz[h];
+        }
+    }
+}
+
+template <class T>
+void launch_gather_state(const View<T>& v, double* out, int* active, cudaStream_t st) {
+    k_gather_state<T><<<(v.n + kBlock - 1) / kBlock, kBlock, 0, st>>>(v, out, active);
+}
+template <class T>
+void launch_gather_forces(const View<T>& v, double* out, cudaStream_t st) {
+    k_gather_forces<T><<<(v.n + kBlock - 1) / kBlock, kBlock, 0, st>>>(v, out);
+}
+template <class T>
+void launch_gather_counts(const View<T>& v, int wall, int* out, cudaStream_t st) {
+    k_gather_counts<T><<<(v.n + kBlock - 1) / kBlock, kBlock, 0, st>>>(v, wall, out);
+}
+template <class T>
+void launch_gather_history(const View<T>& v, int wall, int rows, cudaStream_t st) {
+    k_gather_history<T><<<(v.n + kBlock - 1) / kBlock, kBlock, 0, st>>>(v, wall, rows);
+}
+
+#define GDEM_GATHERS(T)                                                                  \
+    template void launch_gather_state<T>(const View<T>&, double*, int*, cudaStream_t);   \
+    template void launch_gather_forces<T>(const View<T>&, double*, cudaStream_t);        \
+    template void launch_gather_counts<T>(const View<T>&, int, int*, cudaStream_t);      \
+    template void launch_gather_history<T>(const View<T>&, int, int, cudaStream_t);
+GDEM_GATHERS(FP64)
+GDEM_GATHERS(Mixed)
+#undef GDEM_GATHERS
 template void launch_stats<FP64>(const View<FP64>&, double*, int, cudaStream_t);
 template void launch_stats<Mixed>(const View<Mixed>&, double*, int, cudaStream_t);
 template void launch_keys_probe<FP64>(const View<FP64>&, uint32_t*, cudaStream_t);
