@@ -914,38 +914,43 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
 
 // ---------------------------------------------------------------- warp-cooperative
 // The warp-staged pipeline with the particle contacts computed by the whole
-// warp.  Every lane first tests its whole Verlet row (a bit per entry in
-// contact).  Then, kCoopQ contacts per lane at a time, it finds their history
-// slots in row order (the entry's slot hint checked against the key, else a
-// search) and queues them; the warp computes the queued contacts 32 at a
-// time, whoever owns them, and each lane adds its own contacts' results back
-// in row order.  The contact law runs with every lane busy, and its gathers
-// and history loads are in flight together instead of one contact after
-// another.  Shared memory per warp is kept small (two stage buffers and the
-// queue, 6.9 KB) so that five CTAs of four warps share an SM with a large
-// L1 beside them for the neighbour and history gathers: staging the first
-// history-key rows in shared memory as well measured slower (0.463 ms on the
-// 1M bed with three rows, 0.496 with seven, against 0.452 with none).
+// warp, which takes tiles of W = 8, 16 or 32 particles.  Four lanes test a
+// particle's row, eight particles at a time, four entries of each; the entries
+// in contact go, compacted by ballot, into a ring that holds every particle's
+// contacts in row order.  The warp takes 32 of the ring at a time, whoever
+// owns them: slots (the entry's slot hint checked against the key, else a
+// search), contact law and spring, with every lane busy and all of a
+// contact's loads in flight together; each particle's lane then adds its own
+// results in ring order.  Nothing is a loop over one lane's contacts, so a
+// tile's latency is a few dependent loads whatever its contacts are.
+// The kernel is bound by the latency of its gathers.  The form before tested a
+// row per lane and found the slots contact by contact, two dependent loads
+// each, in tiles of 32 only; its step kernel and this one: 2,000 spheres 23.8
+// and 15.0 us, 30,000 31.7 and 22.0, 96,000 in 48 boxes 50 and 34, 250,000
+// (linear law) 101 and 89, 1,000,000 325 and 312.  Shared memory per warp is kept small
+// (two stage buffers and the ring, 7.8 KB) so that five CTAs of four warps
+// share an SM with a large L1 beside them for the neighbour and history
+// gathers.
 constexpr int kCoopWarps = 4;
-constexpr int kCoopQ = 2;
+constexpr int kCoopRows = 4;   // staged row entries: those of the first pass
 
 struct __align__(16) CStage {
     float4 posh[32], posl[32], vel[32], rot[32];
     int nnei[32], nneiw[32], nc[32], ncw[32];
-    int nei[kNeiStageRows][32];
+    int nei[kCoopRows][32];
 };
 static_assert(sizeof(CStage) % 16 == 0, "stage buffers must keep 16-byte alignment");
 
-// The warp's contact queue: a ring the lanes fill kCoopQ contacts each per
-// round and the warp drains 32 at a time (positions grow without bound; the
-// slot of position x is x % kRing).  The queue holds fewer than 32 before a
-// round adds at most 64, so kRing = 96 never overflows.
+// The warp's contact ring (positions grow without bound; position x is kept at
+// x % kRing).  It holds fewer than 32 before 64 more may come, so kRing = 96
+// never overflows.
 constexpr int kRing = 3 * 32;
 struct __align__(16) CQueue {
     int j[kRing];             // partner's storage index
-    int pk[kRing];            // history slot | fresh << 6 | owning lane << 7
+    int pk[kRing];            // 1 + slot hint | owning lane << 6 | row position << 11; its slot once found
     float f[6][32];           // force and torque of each contact of the batch being drained
     unsigned owned[32];       // the positions of a drained batch each lane owns (bit b: head + b)
+    int nc[32];               // history length so far
 };
 
 constexpr size_t kCoopSmem = 2 * kCoopWarps * sizeof(CStage) + kCoopWarps * sizeof(CQueue);
@@ -954,27 +959,28 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
-// Bulk copies of sub-tile `t` into `st` (lane 0): positions, velocities,
-// spins and counts, plus the first Verlet rows when every row k*n + 32t
-// starts 16-byte aligned (n a multiple of 4).  The
-// arrays read only at the end of the sub-tile (low parts, reference
-// positions of the list and inner rows) are prefetched into L2.
+// Bulk copies of the W-particle tile `t` into `st` (lane 0): positions,
+// velocities, spins and counts, plus the first row entries when every row
+// k*n + W t starts 16-byte aligned (n a multiple of 4).  The arrays read only at
+// the end of the tile (low parts, reference positions of the list and inner
+// rows) are prefetched into L2.
+template <int W>
 __device__ __forceinline__ void issue_csub(const View<Mixed>& v, const SBank<Mixed>& A, const PBank<Mixed>& P,
                                            int t, CStage* st, unsigned long long* bar, int nei_rows) {
-    const int base = t * 32;
-    const int cnt = min(32, v.n - base);
+    const int base = t * W;
+    const int cnt = min(W, v.n - base);
     const unsigned b16 = 16u * (unsigned)cnt;
     const unsigned b4 = 4u * (unsigned)((cnt + 3) & ~3);
     mbar_expect_tx(bar, 4u * b16 + (4u + (unsigned)nei_rows) * b4);
     bulk_g2s(st->posh, A.posh + base, b16, bar);
+    for (int k = 0; k < nei_rows; k++) bulk_g2s(st->nei[k], v.nei + (size_t)k * v.n + base, b4, bar);
+    bulk_g2s(st->nnei, v.nnei + base, b4, bar);
+    bulk_g2s(st->rot, A.rot + base, b16, bar);
     bulk_g2s(st->posl, A.posl + base, b16, bar);
     bulk_g2s(st->vel, A.vel + base, b16, bar);
-    bulk_g2s(st->rot, A.rot + base, b16, bar);
-    bulk_g2s(st->nnei, v.nnei + base, b4, bar);
     bulk_g2s(st->nneiw, v.nneiw + base, b4, bar);
     bulk_g2s(st->nc, P.nc + base, b4, bar);
     bulk_g2s(st->ncw, P.ncw + base, b4, bar);
-    for (int k = 0; k < nei_rows; k++) bulk_g2s(st->nei[k], v.nei + (size_t)k * v.n + base, b4, bar);
     bulk_prefetch_l2(A.vell + base, b16);
     bulk_prefetch_l2(A.rotl + base, b16);
     bulk_prefetch_l2(v.refh + base, b16);
@@ -992,9 +998,9 @@ __device__ __forceinline__ void issue_csub(const View<Mixed>& v, const SBank<Mix
 // where it has a contact, so none of it is held in registers across the
 // geometry (which removed the kernel's register spills).  All lanes call it;
 // nw is 0 on inactive lanes.
-template <int MODEL, int WCAP, bool PER>
+template <int MODEL, bool PER>
 __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mixed>& P, const CStage& S, CQueue* que,
-                                           int t, int lane, bool active, int nw, int ncw, Force6& F, unsigned& err) {
+                                           int tile, int lane, bool active, int nw, int ncw, Force6& F, unsigned& err) {
     const int n = v.n;
     const PerX per = per_of<PER>(v);
     int incl = nw;
@@ -1005,9 +1011,9 @@ __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mix
     }
     const int excl = incl - nw;
     const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int i = t * 32 + lane;
+    const int i = tile + lane;
     unsigned long long wtouched = 0ull;
-    int vore[WCAP];
+    int vore[64];  // wall rows hold at most 64
     int nvore = 0;
     for (int base = 0; base < total; base += 32) {
         const int c = base + lane;
@@ -1020,7 +1026,7 @@ __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mix
         int hit = -3, tri = 0;
         float nx = 0.f, ny = 0.f, nz = 0.f, dm = 0.f;
         if (c < total) {
-            tri = __ldg(&v.neiw[(size_t)k * n + t * 32 + ow]);
+            tri = __ldg(&v.neiw[(size_t)k * n + tile + ow]);
             const float4 hiw = S.posh[ow], liw = S.posl[ow];
             const float rm = hiw.w + v.wall_delta;
             float3 qh = make_float3(hiw.x, hiw.y, hiw.z), ql = make_float3(liw.x, liw.y, liw.z);
@@ -1051,7 +1057,7 @@ __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mix
         for (int y = max(excl, base) - base; y < y1; y++) {
             const int fh = __float_as_int(que->f[4][y]);
             if (fh == -3) continue;
-            if (!feature_is_new<WCAP>(fh, vore, nvore)) continue;
+            if (!feature_is_new<64>(fh, vore, nvore)) continue;
             // this lane's state and material, read only where it has a contact
             const float4 hi = S.posh[lane], vi = S.vel[lane], wi = S.rot[lane];
             const Mat mt = own_material<MODEL>(v, P, i, hi.w, vi.w);
@@ -1063,11 +1069,117 @@ __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mix
     if (active) P.ncw[i] = surviving(wtouched, ncw);
 }
 
-template <int MODEL, int WCAP, int MINB, bool PER>
+// The oldest B (<= 32) contacts of the ring: slots, contact law, springs, and
+// the results added to their particles' sums.
+template <int MODEL, bool PER>
+__device__ __forceinline__ void coop_drain(const View<Mixed>& v, const SBank<Mixed>& A, const PBank<Mixed>& P,
+                                           const CStage& S, CQueue* que, int tile, int head, int B, int lane, Force6& F,
+                                           unsigned long long& touched, unsigned& err) {
+    using R = float;
+    const int n = v.n;
+    const PerX per = per_of<PER>(v);
+    const unsigned rmask = v.row_mask;
+    const float4* __restrict__ Aposh = A.posh;
+    const float4* __restrict__ Aposl = A.posl;
+    const float4* __restrict__ Avel = A.vel;
+    const float4* __restrict__ Arot = A.rot;
+    const int x = (head + lane) % kRing;
+    const bool in = lane < B;
+    const int pk = in ? que->pk[x] : 0;
+    const int ow = in ? (pk >> 6) & 31 : 32 + lane;
+    const int j = in ? que->j[x] : 0;
+    const int iow = tile + ow;
+    int slot = (pk & 63) - 1;
+    const int nc0 = in ? S.nc[ow] : 0;
+    if (slot >= nc0) slot = -1;
+    // the spring at the hinted slot is loaded before the key is checked
+    Vec3<R> sp, cp;
+    sp.x = sp.y = sp.z = 0.f;
+    cp.x = cp.y = cp.z = 0.f;
+    bool renew = false;  // the row entry gets a new hint
+    if (in) {
+        if (slot >= 0) {
+            const size_t h = (size_t)slot * n + iow;
+            const int key = P.hid[h];
+            sp.x = P.hx[h]; sp.y = P.hy[h]; sp.z = P.hz[h];
+            cp.x = P.cx[h]; cp.y = P.cy[h]; cp.z = P.cz[h];
+            if (key != j) slot = -1;
+        }
+        if (slot < 0) {
+            renew = true;
+            for (int q = 0; q < nc0; q++)
+                if (P.hid[(size_t)q * n + iow] == j) {
+                    slot = q;
+                    break;
+                }
+            if (slot >= 0) {
+                const size_t h = (size_t)slot * n + iow;
+                sp.x = P.hx[h]; sp.y = P.hy[h]; sp.z = P.hz[h];
+                cp.x = P.cx[h]; cp.y = P.cy[h]; cp.z = P.cz[h];
+            } else {
+                sp.x = sp.y = sp.z = 0.f;
+                cp.x = cp.y = cp.z = 0.f;
+            }
+        }
+    }
+    que->owned[lane] = 0u;
+    const unsigned grp = __match_any_sync(0xffffffffu, ow);
+    // contacts without a slot are appended to their rows in ring order
+    const bool fresh = in && slot < 0;
+    const unsigned fm = __ballot_sync(0xffffffffu, fresh) & grp;
+    if (fresh) {
+        slot = que->nc[ow] + __popc(fm & ((1u << lane) - 1u));
+        if (slot >= v.hist_cap) {
+            slot = -1;
+            err |= 0x4u;
+        } else {
+            P.hid[(size_t)slot * n + iow] = j;
+        }
+    }
+    __syncwarp();
+    if (fresh && lane == __ffs((int)fm) - 1) que->nc[ow] = min(que->nc[ow] + __popc(fm), v.hist_cap);
+    const bool hit = slot >= 0;
+    const unsigned live = __ballot_sync(0xffffffffu, hit) & grp;
+    if (hit) {
+        if (renew && rmask != 0xFFFFFFFFu && slot < 63) v.nei[(size_t)(pk >> 11) * n + iow] = j | ((slot + 1) << kHintShift);
+        que->pk[x] = slot;
+        const float4 hiw = S.posh[ow], liw = S.posl[ow], viw = S.vel[ow], wiw = S.rot[ow];
+        const float4 hjq = __ldg(&Aposh[j]), ljq = __ldg(&Aposl[j]);
+        const float4 vj = __ldg(&Avel[j]), wj = __ldg(&Arot[j]);
+        const size_t h = (size_t)slot * n + iow;
+        const Mat mo = own_material<MODEL>(v, P, iow, hiw.w, viw.w);
+        const Force6 G = pair_force<MODEL>(v, pair_geometry(hiw, liw, hjq, ljq, per), hiw.w, hjq.w, viw, wiw, vj, wj,
+                                           viw.w, mo, sp, cp);
+        P.hx[h] = sp.x; P.hy[h] = sp.y; P.hz[h] = sp.z;
+        P.cx[h] = cp.x; P.cy[h] = cp.y; P.cz[h] = cp.z;
+        que->f[0][lane] = G.fx;
+        que->f[1][lane] = G.fy;
+        que->f[2][lane] = G.fz;
+        que->f[3][lane] = G.mx;
+        que->f[4][lane] = G.my;
+        que->f[5][lane] = G.mz;
+        // the batch positions of each particle, written by its first lane
+        if ((live & ((1u << lane) - 1u)) == 0u) que->owned[ow] = live;
+    }
+    __syncwarp();
+    // each particle's lane adds its results in ring (row) order
+    for (unsigned m = que->owned[lane]; m != 0u; m &= m - 1u) {
+        const int y = __ffs((int)m) - 1;
+        touched |= 1ull << que->pk[(head + y) % kRing];
+        F.fx += que->f[0][y];
+        F.fy += que->f[1][y];
+        F.fz += que->f[2][y];
+        F.mx += que->f[3][y];
+        F.my += que->f[4][y];
+        F.mz += que->f[5][y];
+    }
+    __syncwarp();
+}
+
+template <int MODEL, int G, int MINB, bool PER>
 __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<Mixed> v, cudaGraphConditionalHandle cond, cudaGraphConditionalHandle cond_inner,
                                                                     int use_cond) {
-    using R = float;
-    constexpr int Q = kCoopQ;
+    constexpr int W = 8 * G;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     CStage* stage = reinterpret_cast<CStage*>(smem_raw) + 2 * warp;
@@ -1080,12 +1192,11 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
     const PBank<Mixed> P = v.P[p];
     const float4* __restrict__ Aposh = A.posh;
     const float4* __restrict__ Aposl = A.posl;
-    const float4* __restrict__ Avel = A.vel;
-    const float4* __restrict__ Arot = A.rot;
     const int* __restrict__ nei = v.nei;
     const int n = v.n;
-    const int nsub = (n + 31) / 32;
-    const int nei_rows = (n % 4 == 0) ? min(kNeiStageRows, v.nei_cap) : 0;
+    const int nsub = (n + W - 1) / W;
+    const int nwarps = gridDim.x * kCoopWarps;
+    const int nei_rows = (n % 4 == 0) ? min(kCoopRows, v.nei_cap) : 0;
     const unsigned rmask = v.row_mask;
     const PerX per = per_of<PER>(v);
     unsigned votes = 0u;
@@ -1096,28 +1207,25 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    // sub-tiles are handed out one at a time from a counter, so warps that
-    // meet dense sub-tiles (many contacts, many wall candidates) take fewer
-    int t = 0;
-    if (lane == 0) {
-        t = (int)atomicAdd(&ctl->work, 1u);
-        if (t < nsub) issue_csub(v, A, P, t, &stage[0], &full[warp][0], nei_rows);
-    }
-    t = __shfl_sync(0xffffffffu, t, 0);
+    // a warp's first tile is its own number, the others are handed out one at
+    // a time from a counter, so warps that meet dense tiles (many contacts,
+    // many wall candidates) take fewer
+    int t = blockIdx.x * kCoopWarps + warp;
+    if (lane == 0 && t < nsub) issue_csub<W>(v, A, P, t, &stage[0], &full[warp][0], nei_rows);
     bool timed_out = false;
     int t_it = 0, t_next = nsub;
     for (int it = 0; t < nsub; it++, t = t_next) {
         t_it = it;
         const int b = it & 1;
-        int tn = 0;
-        if (lane == 0) tn = (int)atomicAdd(&ctl->work, 1u);
+        int tn = nsub;
+        if (lane == 0 && nsub > nwarps) tn = nwarps + (int)atomicAdd(&ctl->work, 1u);
         tn = __shfl_sync(0xffffffffu, tn, 0);
         t_next = tn;
         if (lane == 0 && tn < nsub) {
             // the other buffer was last read before the __syncwarp that ended
             // the previous iteration; order those reads before the copy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            issue_csub(v, A, P, tn, &stage[b ^ 1], &full[warp][b ^ 1], nei_rows);
+            issue_csub<W>(v, A, P, tn, &stage[b ^ 1], &full[warp][b ^ 1], nei_rows);
         }
         const bool ok = mbar_wait_bounded(&full[warp][b], (unsigned)(it >> 1) & 1u, v.wait_tries);
         if (__any_sync(0xffffffffu, !ok)) {
@@ -1125,8 +1233,9 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
             break;
         }
         CStage& S = stage[b];
-        const int i = t * 32 + lane;
-        const bool valid = i < n;
+        const int tile = t * W;
+        const int i = tile + lane;  // the particle this lane sums and integrates
+        const bool valid = lane < W && i < n;
         const bool active = valid && S.rot[lane].w == 1.f;
         if (valid && !active) {
             Own o;
@@ -1139,169 +1248,76 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
             freeze_one(v, B, i, o);
         }
         Force6 F = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        int nc = S.nc[lane];
+        if (valid) que->nc[lane] = S.nc[lane];
         unsigned long long touched = 0ull;
-        const int nn = active ? S.nnei[lane] : 0;
-        const int* nei_s = &S.nei[0][lane];
-        // ---- this lane's whole row in one pass, four entries at a time with
-        // their gathers in flight together: a bit per row entry in contact
-        unsigned long long hit_lo = 0ull, hit_hi = 0ull;
-        {
-            const float4 hi = S.posh[lane], li = S.posl[lane];
-            const float delta = v.nb_delta;
-            for (int k0 = 0; k0 < nn; k0 += 4) {
-                int jj[4];
+        // ---- rows: lane 4 a + q tests entries q, q + 4, ... of particle
+        // 8 g + a of each group g
+        int nn[G], most = 0;
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int k = k0 + q;
-                    jj[q] = k < nn ? (int)((unsigned)(k < nei_rows ? nei_s[k * 32] : __ldg(&nei[(size_t)k * n + i])) & rmask)
-                                   : -1;
-                }
-                float4 hj[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (jj[q] >= 0) hj[q] = __ldg(&Aposh[jj[q]]);
-                unsigned hit = 0u;
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    if (jj[q] < 0) continue;
-                    const int h = contact_hint(hi, hj[q], delta, per);
-                    if (h > 0 || (h < 0 && exact_contact(hi, li, hj[q], __ldg(&Aposl[jj[q]]), per))) hit |= 1u << q;
-                }
-                if (k0 < 64)
-                    hit_lo |= (unsigned long long)hit << k0;
-                else
-                    hit_hi |= (unsigned long long)hit << (k0 - 64);
-            }
+        for (int g = 0; g < G; g++) {
+            const int a = 8 * g + (lane >> 2);
+            nn[g] = tile + a < n && S.rot[a].w == 1.f ? S.nnei[a] : 0;
+            most = max(most, nn[g]);
         }
-        // ---- contacts through the ring: each round every lane queues its
-        // next (up to) Q contacts in row order (partner and history slot);
-        // whenever 32 are queued, or none will follow, the warp computes the
-        // oldest 32 with every lane busy, and each lane adds its own results
-        // in queue order, which is its row order
+        most = __reduce_max_sync(0xffffffffu, most);
+        const float delta = v.nb_delta;
         int head = 0, tail = 0;
-        while (true) {
-            static_assert(Q == 2, "a lane queues at most two contacts per round");
-            int cnt = 0;
-            int qj0 = 0, qs0 = 0, qj1 = 0, qs1 = 0;
-#pragma unroll 1
-            for (int q = 0; q < Q && (hit_lo | hit_hi) != 0ull; q++) {
-                int k;
-                if (hit_lo) {
-                    k = __ffsll((long long)hit_lo) - 1;
-                    hit_lo &= hit_lo - 1ull;
-                } else {
-                    k = 64 + __ffsll((long long)hit_hi) - 1;
-                    hit_hi &= hit_hi - 1ull;
-                }
-                const unsigned e = (unsigned)(k < nei_rows ? nei_s[k * 32] : __ldg(&nei[(size_t)k * n + i]));
-                const int j = (int)(e & rmask);
-                // the slot hint of the inner row, checked against the key
-                const int hint = rmask != 0xFFFFFFFFu ? (int)(e >> kHintShift) - 1 : -1;
-                bool fresh = false;
-                int slot;
-                if (hint >= 0 && hint < nc && P.hid[(size_t)hint * n + i] == j) {
-                    slot = hint;
-                } else {
-                    slot = find_slot<Mixed>(P.hid, n, i, nc, j, v.hist_cap, fresh);
-                    if (slot < 0) {
-                        err |= 0x4u;
-                        continue;
-                    }
-                    if (fresh) P.hid[(size_t)slot * n + i] = j;
-                    if (rmask != 0xFFFFFFFFu && slot < 63) v.nei[(size_t)k * n + i] = j | ((slot + 1) << kHintShift);
-                }
-                touched |= 1ull << slot;
-                if (cnt == 0) {
-                    qj0 = j;
-                    qs0 = slot | (fresh ? 64 : 0) | (lane << 7);
-                } else {
-                    qj1 = j;
-                    qs1 = slot | (fresh ? 64 : 0) | (lane << 7);
-                }
-                cnt++;
-            }
-            int excl = cnt;
+        for (int k0 = 0; k0 < most; k0 += 4) {
+            const int k = k0 + (lane & 3);
+            unsigned e[G];
+            float4 hj[G];
 #pragma unroll
-            for (int o2 = 1; o2 < 32; o2 <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, excl, o2);
-                if (lane >= o2) excl += y;
+            for (int g = 0; g < G; g++) {
+                const int a = 8 * g + (lane >> 2);
+                e[g] = 0u;
+                if (k < nn[g])
+                    e[g] = (unsigned)(k < nei_rows ? S.nei[k][a] : __ldg(&nei[(size_t)k * n + tile + a]));
             }
-            const int added = __shfl_sync(0xffffffffu, excl, 31);
-            excl -= cnt;
-            if (cnt > 0) {
-                const int x = (tail + excl) % kRing;
-                que->j[x] = qj0;
-                que->pk[x] = qs0;
+#pragma unroll
+            for (int g = 0; g < G; g++)
+                if (k < nn[g]) hj[g] = __ldg(&Aposh[e[g] & rmask]);
+            unsigned near = 0u;
+#pragma unroll
+            for (int g = 0; g < G; g++) {
+                if (!(k < nn[g])) continue;
+                const int a = 8 * g + (lane >> 2);
+                const float4 hi = S.posh[a];
+                const int c = contact_hint(hi, hj[g], delta, per);
+                if (c > 0 || (c < 0 && exact_contact(hi, S.posl[a], hj[g], __ldg(&Aposl[e[g] & rmask]), per)))
+                    near |= 1u << g;
             }
-            if (cnt > 1) {
-                const int x = (tail + excl + 1) % kRing;
-                que->j[x] = qj1;
-                que->pk[x] = qs1;
-            }
-            tail += added;
-            const bool more = __any_sync(0xffffffffu, (hit_lo | hit_hi) != 0ull);
-            while (tail - head >= 32 || (!more && tail > head)) {
-                const int B = min(32, tail - head);
-                que->owned[lane] = 0u;
-                __syncwarp();
-                // ---- the warp computes the batch [head, head + B)
-                const int x = (head + lane) % kRing;
-                const int sl = lane < B ? que->pk[x] : 0;
-                const int ow = lane < B ? sl >> 7 : 32 + lane;
-                if (lane < B) {
-                    const int j = que->j[x];
-                    const int slot = sl & 63;
-                    const int iow = t * 32 + ow;
-                    const float4 hiw = S.posh[ow], liw = S.posl[ow], viw = S.vel[ow], wiw = S.rot[ow];
-                    const float4 hjq = __ldg(&Aposh[j]), ljq = __ldg(&Aposl[j]);
-                    const float4 vj = __ldg(&Avel[j]), wj = __ldg(&Arot[j]);
-                    const size_t h = (size_t)slot * n + iow;
-                    Vec3<R> sp, cp;
-                    if (sl & 64) {
-                        sp.x = sp.y = sp.z = 0.f;
-                        cp.x = cp.y = cp.z = 0.f;
-                    } else {
-                        sp.x = P.hx[h]; sp.y = P.hy[h]; sp.z = P.hz[h];
-                        cp.x = P.cx[h]; cp.y = P.cy[h]; cp.z = P.cz[h];
+            // two groups at a time into the ring, which is then drained
+#pragma unroll 1
+            for (int g2 = 0; g2 < G; g2 += 2) {
+#pragma unroll
+                for (int u = 0; u < (G < 2 ? 1 : 2); u++) {
+                    const int g = g2 + u;
+                    const bool c = (near >> g) & 1u;
+                    const unsigned m = __ballot_sync(0xffffffffu, c);
+                    if (c) {
+                        unsigned eg = e[u];
+                        if (G > 2 && g2 > 0) eg = e[(2 + u) % G];
+                        const int x = (tail + __popc(m & ((1u << lane) - 1u))) % kRing;
+                        const int hint = rmask != 0xFFFFFFFFu ? (int)(eg >> kHintShift) : 0;
+                        que->j[x] = (int)(eg & rmask);
+                        que->pk[x] = hint | (8 * g + (lane >> 2)) << 6 | k << 11;
                     }
-                    const Mat mo = own_material<MODEL>(v, P, iow, hiw.w, viw.w);
-                    const Force6 G = pair_force<MODEL>(v, pair_geometry(hiw, liw, hjq, ljq, per), hiw.w, hjq.w, viw,
-                                                       wiw, vj, wj, viw.w, mo, sp, cp);
-                    P.hx[h] = sp.x; P.hy[h] = sp.y; P.hz[h] = sp.z;
-                    P.cx[h] = cp.x; P.cy[h] = cp.y; P.cz[h] = cp.z;
-                    que->f[0][lane] = G.fx;
-                    que->f[1][lane] = G.fy;
-                    que->f[2][lane] = G.fz;
-                    que->f[3][lane] = G.mx;
-                    que->f[4][lane] = G.my;
-                    que->f[5][lane] = G.mz;
-                }
-                // the batch positions of each owner: one mask per group of
-                // equal owners, written by the group's first lane
-                const unsigned grp = __match_any_sync(0xffffffffu, ow);
-                if (lane < B && (grp & ((1u << lane) - 1u)) == 0u) que->owned[ow] = grp;
-                __syncwarp();
-                // each lane adds its own results in position (row) order
-                for (unsigned m = que->owned[lane]; m != 0u; m &= m - 1u) {
-                    const int y = __ffs((int)m) - 1;
-                    F.fx += que->f[0][y];
-                    F.fy += que->f[1][y];
-                    F.fz += que->f[2][y];
-                    F.mx += que->f[3][y];
-                    F.my += que->f[4][y];
-                    F.mz += que->f[5][y];
+                    tail += __popc(m);
                 }
                 __syncwarp();
-                head += B;
+                const bool last = k0 + 4 >= most && g2 + 2 >= G;
+                while (tail - head >= 32 || (last && tail > head)) {
+                    const int cnt = min(32, tail - head);
+                    coop_drain<MODEL, PER>(v, A, P, S, que, tile, head, cnt, lane, F, touched, err);
+                    head += cnt;
+                }
             }
-            if (!more) break;
         }
         // ---- wall contacts, the geometry over the whole warp
-        coop_walls<MODEL, WCAP, PER>(v, P, S, que, t, lane, active, active ? S.nneiw[lane] : 0, S.ncw[lane], F, err);
+        coop_walls<MODEL, PER>(v, P, S, que, tile, lane, active, active ? S.nneiw[lane] : 0, S.ncw[lane], F, err);
         if (active) {
             const Mat mt = own_material<MODEL>(v, P, i, S.posh[lane].w, S.vel[lane].w);
-            P.nc[i] = surviving(touched, nc);
+            P.nc[i] = surviving(touched, que->nc[lane]);
             Own o;
             o.wi = S.rot[lane];
             o.hi = S.posh[lane];
@@ -1355,25 +1371,25 @@ void* wtma_kernel(int wall_cap) {
     }
     return fn;
 }
-template <int MODEL, int MINB, bool PER>
-void* coop_kernel_minb(int wall_cap) {
-    void* fn = wall_cap <= 16   ? (void*)k_step_mixed_coop<MODEL, 16, MINB, PER>
-               : wall_cap <= 32 ? (void*)k_step_mixed_coop<MODEL, 32, MINB, PER>
-                                : (void*)k_step_mixed_coop<MODEL, 64, MINB, PER>;
-    static bool configured[3] = {false, false, false};
-    const int slot = wall_cap <= 16 ? 0 : (wall_cap <= 32 ? 1 : 2);
-    if (!configured[slot]) {
+template <int MODEL, int G, int MINB, bool PER>
+void* coop_kernel_of() {
+    void* fn = (void*)k_step_mixed_coop<MODEL, G, MINB, PER>;
+    static bool configured = false;
+    if (!configured) {
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoopSmem);
-        configured[slot] = true;
+        configured = true;
     }
     return fn;
 }
+// `g`: tile width over 8 (1, 2 or 4); the narrow tiles, and a periodic x,
+// exist at the default occupancy only
 template <int MODEL>
-void* coop_kernel(int wall_cap, int minb, bool per) {
-    if (per) return coop_kernel_minb<MODEL, 5, true>(wall_cap);
-    return minb == 4 ? coop_kernel_minb<MODEL, 4, false>(wall_cap)
-                     : (minb == 6 ? coop_kernel_minb<MODEL, 6, false>(wall_cap)
-                                  : coop_kernel_minb<MODEL, 5, false>(wall_cap));
+void* coop_kernel(int g, int minb, bool per) {
+    if (g == 1) return per ? coop_kernel_of<MODEL, 1, 5, true>() : coop_kernel_of<MODEL, 1, 5, false>();
+    if (g == 2) return per ? coop_kernel_of<MODEL, 2, 5, true>() : coop_kernel_of<MODEL, 2, 5, false>();
+    if (per) return coop_kernel_of<MODEL, 4, 5, true>();
+    return minb == 4 ? coop_kernel_of<MODEL, 4, 4, false>()
+                     : (minb == 6 ? coop_kernel_of<MODEL, 4, 6, false>() : coop_kernel_of<MODEL, 4, 5, false>());
 }
 // Kernel and occupancy: the engine's settings, else the environment
 // (GDEM_MIXED_KERNEL=staged|direct, GDEM_COOP_MINB, GDEM_MIXED_MINB), else the
@@ -1401,12 +1417,20 @@ StepLaunch step_launch(const View<Mixed>& v, int reserve) {
         static const int env_minb = env_int("GDEM_COOP_MINB", 5);
         const int minb = v.occupancy > 0 ? v.occupancy : env_minb;
         const bool per = v.per_x != 0;
-        void* fn = v.mat.model == 1 ? coop_kernel<1>(v.wall_cap, minb, per) : coop_kernel<0>(v.wall_cap, minb, per);
+        // Tile width: the narrowest at which every tile still has a resident
+        // warp of its own (20 per SM), since a tile's latency grows with its
+        // particles while the chip is not full; full tiles once it is.  Step
+        // of a Hertz-Mindlin bed at 8 / 16 / 32 to a tile: 16,000 spheres
+        // 28 / 29 / 36 us, 24,000 31 / 33 / 37, 30,000 37 / 32 / 38, 40,000
+        // 39 / 33 / 37, 50,000 42 / 40 / 38, 80,000 53 / 47 / 42.
+        const int warps = 20 * sm_count();
+        const int g = v.n <= 8 * warps ? 1 : (v.n <= 16 * warps ? 2 : 4);
+        void* fn = v.mat.model == 1 ? coop_kernel<1>(g, minb, per) : coop_kernel<0>(g, minb, per);
         const size_t smem = kCoopSmem;
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kCoopWarps * 32, smem);
         if (per_sm < 1) per_sm = 1;
-        const int nsub = (v.n + 31) / 32;
+        const int nsub = (v.n + 8 * g - 1) / (8 * g);
         const int need = (nsub + kCoopWarps - 1) / kCoopWarps;
         // GDEM_COOP_RESERVE overrides a nonzero reserve (tuning)
         static const int env_reserve = env_int("GDEM_COOP_RESERVE", -1);

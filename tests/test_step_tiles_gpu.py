@@ -89,3 +89,45 @@ def test_fp64_tiles_match_the_oracle(n, model):
 def test_fp64_sphere_with_many_contacts_matches_the_oracle(model):
     s = _same(_crowded(7), model, (1, 2, 60), nei_capacity=128, hist_capacity=64, wall_capacity=64)
     assert s["n_contacts"] > 50
+
+
+def _mixed_state(sc, model, steps, kernel, **kw):
+    from gpudem_gb300 import engine
+    E = engine.Engine(sc, precision="mixed", model=model, mixed_kernel=kernel, store_forces=True, **kw)
+    E.step(steps)
+    st = E.export(history=True, forces=True)
+    s = E.stats()
+    assert s["error_word"] == 0
+    E.close()
+    return st, s
+
+
+@pytest.mark.parametrize("n", [1, 7, 9, 33, 130, 2049, 24_400, 49_001])
+@pytest.mark.parametrize("model", ["linear", "hertz_mindlin"])
+def test_mixed_tiles_match_one_thread_per_particle(n, model):
+    sc = _dense(n, 300 + n, 0.05 if n % 2 else 0.0)
+    a, s = _mixed_state(sc, model, 40, 1)
+    b, _ = _mixed_state(sc, model, 40, 3)
+    # the Hertz-Mindlin law rounds alike in both kernels; the linear law's
+    # multiply-adds are contracted differently, a few FP32 ulps (5e-7) of the
+    # forces, which move a sphere by some 1e-5 m in these 40 steps: 3e-9 r
+    if model == "hertz_mindlin":
+        for nm in a:
+            assert np.array_equal(a[nm], b[nm]), nm
+    else:
+        for nm in ("isActive", "numCont", "numContWall", "indHis", "indHisWall"):
+            assert np.array_equal(a[nm], b[nm]), nm
+        assert np.max(np.abs(a["x"] - b["x"])) <= 1e-7 * sc.r.min()
+    if n >= 130:
+        assert s["n_contacts"] > n and s["n_wall_contacts"] > 0
+
+
+@pytest.mark.parametrize("inner_skin", [0.0, -1.0])
+def test_mixed_sphere_with_many_contacts(inner_skin):
+    sc = _crowded(9)
+    kw = dict(nei_capacity=128, hist_capacity=64, wall_capacity=64, inner_skin=inner_skin)
+    a, s = _mixed_state(sc, "hertz_mindlin", 30, 1, **kw)
+    b, _ = _mixed_state(sc, "hertz_mindlin", 30, 3, **kw)
+    for nm in a:
+        assert np.array_equal(a[nm], b[nm]), nm
+    assert s["n_contacts"] > 50
