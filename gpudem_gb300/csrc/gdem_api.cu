@@ -465,76 +465,140 @@ struct Impl : EngineBase {
         return s;
     }
 
-    int build_graph(int steps, cudaGraphExec_t* out) {
+    // A conditional node (IF, WHILE) in `g` after `deps`; its body graph.
+    cudaError_t add_conditional(cudaGraph_t g, const cudaGraphNode_t* deps, size_t ndeps, cudaGraphConditionalHandle h,
+                                cudaGraphConditionalNodeType type, cudaGraphNode_t* node, cudaGraph_t* body) {
+        cudaGraphNodeParams cp = {};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = type;
+        cp.conditional.size = 1;
+        const cudaError_t e = cudaGraphAddNode(node, g, deps, nullptr, ndeps, &cp);
+        if (e == cudaSuccess) *body = cp.conditional.phGraph_out[0];
+        return e;
+    }
+
+    // What `launch` enqueues on the stream, captured as the nodes of `body`.
+    template <class F>
+    cudaError_t capture_into(cudaGraph_t body, F launch) {
+        cudaError_t e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (e != cudaSuccess) return e;
+        launch();
+        cudaGraph_t captured;
+        return cudaStreamEndCapture(st, &captured);
+    }
+
+    // The step kernel (and beside it the mesh tree rebuild, when asked) after
+    // `dep`; the nodes that end the step.
+    int add_step(cudaGraph_t g, const cudaGraphNode_t* dep, View<T>& vs, const StepLaunch& L, bool tree,
+                 cudaGraphConditionalHandle cond, cudaGraphConditionalHandle inner, int use_cond,
+                 cudaGraphNode_t ends[2], int* nends) {
+        void* args[4] = {(void*)&vs, (void*)&cond, (void*)&inner, (void*)&use_cond};
+        cudaKernelNodeParams kp = {};
+        kp.func = L.fn;
+        kp.gridDim = L.grid;
+        kp.blockDim = L.block;
+        kp.sharedMemBytes = (unsigned)L.smem;
+        kp.kernelParams = args;
+        CKE(cudaGraphAddKernelNode(&ends[0], g, dep, dep ? 1 : 0, &kp));
+        *nends = 1;
+        if (tree) {
+            // the step kernel reads no part of the tree; the list rebuild that
+            // reads it waits for both
+            cudaGraph_t bg;
+            CKE(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            launch_bvh_rebuild(*mesh, st);
+            CKE(cudaStreamEndCapture(st, &bg));
+            CKE(cudaGraphAddChildGraphNode(&ends[1], g, dep, dep ? 1 : 0, bg));
+            cudaGraphDestroy(bg);
+            *nends = 2;
+        }
+        return GDEM_OK;
+    }
+
+    // One step: the step kernel, then the rebuilds it asked for.
+    int build_single(cudaGraphExec_t* out) {
         cudaGraph_t g;
         CKE(cudaGraphCreate(&g, 0));
-        cudaGraphNode_t prev = nullptr;
         View<T> vs = sv();
-        const bool tree_branch = d.bvh_every_step && mesh && mesh->ntri > 0;
-        // the tree rebuild's kernels get CTA slots of their own beside the
-        // persistent step kernel, instead of waiting for it to drain
-        const StepLaunch L = step_launch(vs, tree_branch ? kTreeReserve : 0);
-        for (int k = 0; k < steps; k++) {
-            // every handle must belong to a conditional node: the inner-rows
-            // handle exists only with inner rows (else the kernel gets hnd twice
-            // and leaves the second alone)
-            cudaGraphConditionalHandle hnd, hin;
-            CKE(cudaGraphConditionalHandleCreate(&hnd, g, 0, cudaGraphCondAssignDefault));
-            hin = hnd;
-            if (v.inner_on) CKE(cudaGraphConditionalHandleCreate(&hin, g, 0, cudaGraphCondAssignDefault));
-            int use_cond = v.inner_on ? 3 : 1;
-            void* args[4] = {(void*)&vs, (void*)&hnd, (void*)&hin, (void*)&use_cond};
-            cudaKernelNodeParams kp = {};
-            kp.func = L.fn;
-            kp.gridDim = L.grid;
-            kp.blockDim = L.block;
-            kp.sharedMemBytes = (unsigned)L.smem;
-            kp.kernelParams = args;
-            cudaGraphNode_t sn[2];
-            int nsn = 1;
-            CKE(cudaGraphAddKernelNode(&sn[0], g, prev ? &prev : nullptr, prev ? 1 : 0, &kp));
-            if (tree_branch) {
-                // the mesh tree rebuild runs beside the step kernel, which
-                // reads no part of the tree; the list rebuild that reads it
-                // waits for both
-                cudaGraph_t bg;
-                CKE(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                launch_bvh_rebuild(*mesh, st);
-                CKE(cudaStreamEndCapture(st, &bg));
-                CKE(cudaGraphAddChildGraphNode(&sn[1], g, prev ? &prev : nullptr, prev ? 1 : 0, bg));
-                cudaGraphDestroy(bg);
-                nsn = 2;
+        const bool tree = d.bvh_every_step && mesh && mesh->ntri > 0;
+        const StepLaunch L = step_launch(vs, tree ? kTreeReserve : 0);
+        // every handle must belong to a conditional node: the inner-rows
+        // handle exists only with inner rows (else the kernel gets the lists'
+        // handle twice and leaves the second alone)
+        cudaGraphConditionalHandle hl, hi;
+        CKE(cudaGraphConditionalHandleCreate(&hl, g, 0, cudaGraphCondAssignDefault));
+        hi = hl;
+        if (v.inner_on) CKE(cudaGraphConditionalHandleCreate(&hi, g, 0, cudaGraphCondAssignDefault));
+        cudaGraphNode_t ends[2], node;
+        int nends = 0;
+        if (int rc = add_step(g, nullptr, vs, L, tree, hl, hi, v.inner_on ? kCondLists | kCondInner : kCondLists, ends,
+                              &nends))
+            return rc;
+        cudaGraph_t body;
+        CKE(add_conditional(g, ends, nends, hl, cudaGraphCondTypeIf, &node, &body));
+        CKE(capture_into(body, [&] { launch_rebuild(v, st, /*force=*/1); }));
+        if (v.inner_on) {
+            // new inner rows when some particle moved half the inner skin
+            // (after a list rebuild, its own body already made them)
+            const cudaGraphNode_t prev = node;
+            CKE(add_conditional(g, &prev, 1, hi, cudaGraphCondTypeIf, &node, &body));
+            CKE(capture_into(body, [&] { launch_inner(v, st); }));
+        }
+        CKE(cudaGraphInstantiate(out, g, 0));
+        cudaGraphDestroy(g);
+        return GDEM_OK;
+    }
+
+    // Any number of steps (ctl->remaining): while steps remain, first the rows
+    // that the step before asked for, then a chain of K step kernels with no
+    // condition between them (chain_passes in gdem_step.cuh).  With condition
+    // nodes after every step a step took 10 us more than its kernel; steps of
+    // a bed before and now: 100 spheres in FP64 34 and 27 us, mixed 2,000 25
+    // and 15, 30,000 33 and 20, 250,000 102 and 89.  Chains of 16 and 32 gain
+    // under 1 us on beds and lose 5 and 14 us a step where every third step
+    // asks for new rows (a pour): each step behind it passes at 2 us.
+    int build_loop(cudaGraphExec_t* out) {
+        cudaGraph_t g, body, any, sub;
+        CKE(cudaGraphCreate(&g, 0));
+        View<T> vs = sv();
+        const bool tree = d.bvh_every_step && mesh && mesh->ntri > 0;
+        const StepLaunch L = step_launch(vs, tree ? kTreeReserve : 0);
+        const int inner = v.inner_on;
+        cudaGraphConditionalHandle hw, ha, hl, hi = 0;
+        CKE(cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
+        cudaGraphNode_t node, prev;
+        CKE(add_conditional(g, nullptr, 0, hw, cudaGraphCondTypeWhile, &node, &body));
+        CKE(cudaGraphConditionalHandleCreate(&ha, body, 0, cudaGraphCondAssignDefault));
+        CKE(capture_into(body, [&] { launch_chain_any(v.ctl, inner, ha, st); }));
+        size_t cnt = 1;
+        CKE(cudaGraphGetNodes(body, &prev, &cnt));
+        CKE(add_conditional(body, &prev, 1, ha, cudaGraphCondTypeIf, &node, &any));
+        prev = node;
+        {
+            cudaGraphNode_t q, r;
+            CKE(cudaGraphConditionalHandleCreate(&hl, any, 0, cudaGraphCondAssignDefault));
+            if (inner) CKE(cudaGraphConditionalHandleCreate(&hi, any, 0, cudaGraphCondAssignDefault));
+            CKE(capture_into(any, [&] { launch_chain_which(v.ctl, inner, hl, hi, st); }));
+            cnt = 1;
+            CKE(cudaGraphGetNodes(any, &q, &cnt));
+            CKE(add_conditional(any, &q, 1, hl, cudaGraphCondTypeIf, &r, &sub));
+            CKE(capture_into(sub, [&] { launch_rebuild(v, st, /*force=*/1); }));
+            if (inner) {
+                CKE(add_conditional(any, &r, 1, hi, cudaGraphCondTypeIf, &q, &sub));
+                CKE(capture_into(sub, [&] { launch_inner(v, st); }));
             }
-            cudaGraphNodeParams cp = {};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = hnd;
-            cp.conditional.type = cudaGraphCondTypeIf;
-            cp.conditional.size = 1;
-            cudaGraphNode_t cn;
-            CKE(cudaGraphAddNode(&cn, g, sn, nullptr, nsn, &cp));
-            cudaGraph_t body = cp.conditional.phGraph_out[0];
-            CKE(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
-                                              cudaStreamCaptureModeThreadLocal));
-            launch_rebuild(v, st, /*force=*/1);
-            cudaGraph_t captured;
-            CKE(cudaStreamEndCapture(st, &captured));
-            prev = cn;
-            if (v.inner_on) {
-                // new inner rows when some particle moved half the inner skin
-                // (after a list rebuild, its own body already made them)
-                cudaGraphNodeParams ip = {};
-                ip.type = cudaGraphNodeTypeConditional;
-                ip.conditional.handle = hin;
-                ip.conditional.type = cudaGraphCondTypeIf;
-                ip.conditional.size = 1;
-                cudaGraphNode_t in;
-                CKE(cudaGraphAddNode(&in, g, &prev, nullptr, 1, &ip));
-                CKE(cudaStreamBeginCaptureToGraph(st, ip.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                  cudaStreamCaptureModeThreadLocal));
-                launch_inner(v, st);
-                cudaGraph_t cap2;
-                CKE(cudaStreamEndCapture(st, &cap2));
-                prev = in;
+        }
+        for (int k = 0; k < K; k++) {
+            cudaGraphNode_t ends[2];
+            int nends = 0;
+            if (int rc = add_step(body, &prev, vs, L, tree, hw, hw, kChained | (k == K - 1 ? kChainEnd : 0), ends, &nends))
+                return rc;
+            prev = ends[0];
+            if (nends == 2) {
+                // the next step waits for both
+                CKE(cudaGraphAddEmptyNode(&node, body, ends, 2));
+                prev = node;
             }
         }
         CKE(cudaGraphInstantiate(out, g, 0));
@@ -839,15 +903,23 @@ struct Impl : EngineBase {
             CKE(cudaGetLastError());
             return GDEM_OK;
         }
-        if (!gK) {
-            int rc = build_graph(K, &gK);
-            if (rc) return rc;
-            rc = build_graph(1, &g1);
-            if (rc) return rc;
+        // Steps that pass still rebuild the mesh tree beside them (80 us on the
+        // 1M bed, 2 us without a tree), so with a tree the loop takes whole
+        // chains only.
+        const bool tree = d.bvh_every_step && mesh && mesh->ntri > 0;
+        const int looped = tree ? nsteps - nsteps % K : (nsteps > 1 ? nsteps : 0);
+        if (looped > 0) {
+            if (!gK)
+                if (int rc = build_loop(&gK)) return rc;
+            launch_chain_start(v.ctl, looped, st);
+            CKE(cudaGetLastError());
+            CKE(cudaGraphLaunch(gK, st));
         }
-        const int full = nsteps / K, rest = nsteps % K;
-        for (int q = 0; q < full; q++) CKE(cudaGraphLaunch(gK, st));
-        for (int q = 0; q < rest; q++) CKE(cudaGraphLaunch(g1, st));
+        for (int q = looped; q < nsteps; q++) {
+            if (!g1)
+                if (int rc = build_single(&g1)) return rc;
+            CKE(cudaGraphLaunch(g1, st));
+        }
         return GDEM_OK;
     }
 

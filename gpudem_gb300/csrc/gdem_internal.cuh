@@ -107,7 +107,9 @@ struct Ctl {
     int lists_valid;
     unsigned work;            // next sub-tile of the persistent step kernel (0 between steps)
     unsigned irefresh;        // mixed mode: the inner rows are to be rebuilt
-    unsigned pad;
+    unsigned hold;            // chained steps: rows are to be rebuilt, or no step remains: the rest of the chain passes
+    int remaining;            // chained steps still to take
+    int pad;
     unsigned long long inner_builds;
     unsigned wall_alloc;      // entries taken from the cell wall-candidate buffer (this rebuild)
     unsigned ncell_list;      // occupied cells listed in cell_list (this rebuild)
@@ -598,6 +600,16 @@ __device__ __forceinline__ void split2(double x, float& hi, float& lo) {
 void launch_step(const View<FP64>& v, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond);
 void launch_step(const View<Mixed>& v, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond);
 // The step kernel a launch uses and its launch shape.
+// What a step kernel does beside the step (its use_cond argument): set the list
+// rebuild's condition, the inner rows' condition; belong to a chain (pass when
+// ctl->hold is set, count ctl->remaining down); end one (set the loop condition).
+constexpr int kCondLists = 1, kCondInner = 2, kChained = 4, kChainEnd = 8;
+// Start of `steps` chained steps; the chain's own opening (conditions of the
+// rebuilds: `any`, then `lists` and `inner` apart).
+void launch_chain_start(Ctl* ctl, int steps, cudaStream_t st);
+void launch_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaStream_t st);
+void launch_chain_which(Ctl* ctl, int inner, cudaGraphConditionalHandle lists, cudaGraphConditionalHandle in,
+                        cudaStream_t st);
 struct StepLaunch {
     void* fn;
     dim3 grid, block;

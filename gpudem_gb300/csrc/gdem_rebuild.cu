@@ -1033,6 +1033,27 @@ __global__ void __launch_bounds__(kBlock) k_inner(View<T> v) {
     }
 }
 
+// ===================================================================== step chains
+__global__ void k_chain_start(Ctl* ctl, int steps) { ctl->remaining = steps; }
+__global__ void k_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any) {
+    cudaGraphSetConditional(any, ctl->refresh != 0u || (inner && ctl->irefresh != 0u) ? 1u : 0u);
+    ctl->hold = ctl->remaining <= 0 ? 1u : 0u;
+}
+__global__ void k_chain_which(Ctl* ctl, int inner, cudaGraphConditionalHandle lists, cudaGraphConditionalHandle in) {
+    const unsigned r = ctl->refresh;
+    cudaGraphSetConditional(lists, r != 0u ? 1u : 0u);
+    // a list rebuild makes new inner rows itself
+    if (inner) cudaGraphSetConditional(in, r == 0u && ctl->irefresh != 0u ? 1u : 0u);
+}
+void launch_chain_start(Ctl* ctl, int steps, cudaStream_t st) { k_chain_start<<<1, 1, 0, st>>>(ctl, steps); }
+void launch_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaStream_t st) {
+    k_chain_any<<<1, 1, 0, st>>>(ctl, inner, any);
+}
+void launch_chain_which(Ctl* ctl, int inner, cudaGraphConditionalHandle lists, cudaGraphConditionalHandle in,
+                        cudaStream_t st) {
+    k_chain_which<<<1, 1, 0, st>>>(ctl, inner, lists, in);
+}
+
 static inline int grid_for(int n) { return (n + kBlock - 1) / kBlock; }
 
 template <class T>

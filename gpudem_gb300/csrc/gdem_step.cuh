@@ -18,6 +18,37 @@ inline int sm_count() {
     return c;
 }
 
+// A chained step kernel's first question: does it pass?  Several steps run one
+// after another in a graph without asking the rebuild conditions in between
+// (10 us a step); when a step asks for new rows, those behind it in the chain
+// pass, the rows are rebuilt, and the loop around the chain goes on with the
+// steps that remain (once more for the rows alone, when the last step asked).  `hold` is written by the last CTA of an earlier kernel
+// only, so every CTA of a kernel sees the same answer.
+__device__ __forceinline__ bool chain_passes(Ctl* ctl, int use_cond, int inner, cudaGraphConditionalHandle loop) {
+    if (!(use_cond & kChained) || ctl->hold == 0u) return false;
+    if ((use_cond & kChainEnd) && blockIdx.x == 0 && threadIdx.x == 0)
+        cudaGraphSetConditional(loop, ctl->remaining > 0 || ctl->refresh || (inner && ctl->irefresh) ? 1u : 0u);
+    return true;
+}
+
+// End of a step, by one thread of its last CTA: the bank flip, the step count,
+// and the graph's conditions.
+__device__ __forceinline__ void step_close(Ctl* ctl, int s, int use_cond, int inner, cudaGraphConditionalHandle cond,
+                                           cudaGraphConditionalHandle cond_inner) {
+    ctl->s = s ^ 1;
+    ctl->steps += 1ull;
+    if (!use_cond) return;
+    const unsigned r = atomicAdd(&ctl->refresh, 0u), ri = inner ? atomicAdd(&ctl->irefresh, 0u) : 0u;
+    if (use_cond & kCondLists) cudaGraphSetConditional(cond, r ? 1u : 0u);
+    if (use_cond & kCondInner) cudaGraphSetConditional(cond_inner, ri ? 1u : 0u);
+    if (use_cond & kChained) {
+        const int left = ctl->remaining - 1;
+        ctl->remaining = left;
+        ctl->hold = (r | ri) != 0u || left <= 0 ? 1u : 0u;
+        if (use_cond & kChainEnd) cudaGraphSetConditional(cond, left > 0 || (r | ri) != 0u ? 1u : 0u);
+    }
+}
+
 template <typename R>
 struct Vec3 {
     R x, y, z;

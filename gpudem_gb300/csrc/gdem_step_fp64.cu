@@ -569,6 +569,7 @@ __global__ void __launch_bounds__(32) k_step64(View<FP64> v, cudaGraphConditiona
                                                int use_cond) {
     __shared__ Warp64 S;
     Ctl* ctl = v.ctl;
+    if (chain_passes(ctl, use_cond, 0, cond)) return;
     const int s = ctl->s, p = ctl->p;
     bool refresh = false;
     unsigned err = 0u;
@@ -578,10 +579,7 @@ __global__ void __launch_bounds__(32) k_step64(View<FP64> v, cudaGraphConditiona
     if (last_block(&ctl->done[0])) {
         if (threadIdx.x == 0) {
             ctl->done[0] = 0;
-            ctl->s = s ^ 1;
-            ctl->steps += 1ull;
-            const unsigned r = atomicAdd(&ctl->refresh, 0u);
-            if (use_cond) cudaGraphSetConditional(cond, r ? 1u : 0u);
+            step_close(ctl, s, use_cond, 0, cond, cond);
         }
     }
 }

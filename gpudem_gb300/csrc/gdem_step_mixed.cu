@@ -238,9 +238,8 @@ __device__ __forceinline__ float wall_overlap(float3 ph, float3 pl, float rh, fl
 constexpr unsigned kVoteLists = 1u, kVoteInner = 2u;
 
 // End of a step kernel: refresh votes, error bits, and in the last CTA the
-// bank flip, the step count and the graph's rebuild conditions (list rebuild;
-// inner rows, when use_cond has bit 1).
-__device__ __forceinline__ void step_epilogue(Ctl* ctl, int s, unsigned votes, unsigned err,
+// end of the step.
+__device__ __forceinline__ void step_epilogue(Ctl* ctl, int s, int inner, unsigned votes, unsigned err,
                                               cudaGraphConditionalHandle cond, cudaGraphConditionalHandle ci,
                                               int use_cond) {
     const unsigned wv = __reduce_or_sync(0xffffffffu, votes);
@@ -253,11 +252,7 @@ __device__ __forceinline__ void step_epilogue(Ctl* ctl, int s, unsigned votes, u
         if (threadIdx.x == 0) {
             ctl->done[0] = 0;
             ctl->work = 0;
-            ctl->s = s ^ 1;
-            ctl->steps += 1ull;
-            const unsigned r = atomicAdd(&ctl->refresh, 0u);
-            if (use_cond) cudaGraphSetConditional(cond, r ? 1u : 0u);
-            if (use_cond & 2) cudaGraphSetConditional(ci, atomicAdd(&ctl->irefresh, 0u) ? 1u : 0u);
+            step_close(ctl, s, use_cond, inner, cond, ci);
         }
     }
 }
@@ -728,6 +723,7 @@ template <int MODEL, int WCAP, int MINB, bool PER>
 __global__ void __launch_bounds__(kBlock, MINB) k_step_mixed(View<Mixed> v, cudaGraphConditionalHandle cond, cudaGraphConditionalHandle cond_inner,
                                                             int use_cond) {
     Ctl* ctl = v.ctl;
+    if (chain_passes(ctl, use_cond, v.inner_on, cond)) return;
     const int s = ctl->s, p = ctl->p;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const SBank<Mixed> A = v.S[s];
@@ -750,7 +746,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_step_mixed(View<Mixed> v, cuda
         o.ncw = P.ncw[i];
         step_one<MODEL, WCAP, PER>(v, A, B, P, i, o, votes, err);
     }
-    step_epilogue(ctl, s, votes, err, cond, cond_inner, use_cond);
+    step_epilogue(ctl, s, v.inner_on, votes, err, cond, cond_inner, use_cond);
 }
 
 // ---------------------------------------------------------------- bulk copies
@@ -847,6 +843,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
     WStage* stage = reinterpret_cast<WStage*>(smem_raw) + 2 * warp;
     __shared__ __align__(8) unsigned long long full[kWarps][2];
     Ctl* ctl = v.ctl;
+    if (chain_passes(ctl, use_cond, v.inner_on, cond)) return;
     const int s = ctl->s, p = ctl->p;
     const SBank<Mixed> A = v.S[s];
     const SBank<Mixed> B = v.S[s ^ 1];
@@ -909,7 +906,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
         }
         __syncwarp();
     }
-    step_epilogue(ctl, s, votes, err, cond, cond_inner, use_cond);
+    step_epilogue(ctl, s, v.inner_on, votes, err, cond, cond_inner, use_cond);
 }
 
 // ---------------------------------------------------------------- warp-cooperative
@@ -1186,6 +1183,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
     CQueue* que = reinterpret_cast<CQueue*>(smem_raw + 2 * kCoopWarps * sizeof(CStage)) + warp;
     __shared__ __align__(8) unsigned long long full[kCoopWarps][2];
     Ctl* ctl = v.ctl;
+    if (chain_passes(ctl, use_cond, v.inner_on, cond)) return;
     const int s = ctl->s, p = ctl->p;
     const SBank<Mixed> A = v.S[s];
     const SBank<Mixed> B = v.S[s ^ 1];
@@ -1339,7 +1337,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
         }
         __syncwarp();
     }
-    step_epilogue(ctl, s, votes, err, cond, cond_inner, use_cond);
+    step_epilogue(ctl, s, v.inner_on, votes, err, cond, cond_inner, use_cond);
 }
 
 namespace {
