@@ -46,3 +46,36 @@ def test_chains_take_the_same_steps(precision, tree):
             assert np.array_equal(st[nm], ref[nm]), (chain, nm)
         for a, b in zip(ls, rl):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_graphs_follow_a_new_import_and_new_materials(precision):
+    """An engine that was stepped before takes the same steps after a new import
+    (the same grid, another one, per-particle materials) as a new engine."""
+    from dataclasses import replace
+
+    from gpudem_gb300 import engine
+    a = _shower(600, 5)
+    b = replace(a, r=a.r * 0.97, v=-a.v)       # another r_max: another grid and skin
+    rng = np.random.default_rng(8)
+    mu, e = rng.uniform(0.2, 0.6, a.n), rng.uniform(0.3, 0.8, a.n)
+
+    def run(E, sc, mats):
+        E.import_particles(sc)
+        if mats:
+            E.set_particle_materials(mu, e)
+        E.step(29)
+        st, s = E.export(history=True), E.stats()
+        assert s["error_word"] == 0 and s["steps"] == 29
+        return st
+
+    kw = dict(precision=precision, model="hertz_mindlin")
+    E = engine.Engine(a, **kw)
+    for sc, mats in ((a, False), (a, True), (b, True), (b, False), (a, False)):
+        got = run(E, sc, mats)
+        F = engine.Engine(sc, **kw)
+        want = run(F, sc, mats)
+        F.close()
+        for nm in want:
+            assert np.array_equal(got[nm], want[nm]), (mats, nm)
+    E.close()
