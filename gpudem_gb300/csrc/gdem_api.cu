@@ -347,7 +347,6 @@ struct Impl : EngineBase {
             A.add(&v.ftmp, (size_t)6 * n);
         }
         if (T::mixed) A.add(&v.inv, n);
-        A.add(&v.where, n);
         // cell wall-candidate lists: a count and a base per cell start, and
         // the shared buffer (4 entries per particle; a cell that finds it
         // full falls back to the per-particle tree traversal)
