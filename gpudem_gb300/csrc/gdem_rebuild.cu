@@ -171,9 +171,64 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(
     }
 }
 
+// The same stable sort of up to kSortSmall pairs in one launch, by one CTA: a
+// bitonic network over key << 32 | position in shared memory (equal keys keep
+// their order by position).  Strides up to 32 stay within the 64 elements that a
+// warp holds, so 27 of the 78 stages of 4,096 elements wait for the whole CTA.
+// A sort this small is bound by launches and latency: eight launches of the
+// radix passes took TODO us, this one TODO.
+constexpr int kSortSmall = 4096;
+
+__global__ void __launch_bounds__(1024) k_sort_small(uint32_t* __restrict__ keys, int* __restrict__ vals, int n,
+                                                     int padded, const Ctl* ctl, int gated) {
+    __shared__ unsigned long long a[kSortSmall];
+    if (gated && ctl->refresh == 0u) return;
+    const int t = threadIdx.x;
+    int val[kSortSmall / 1024];
+    for (int i = t; i < padded; i += 1024)
+        a[i] = i < n ? (unsigned long long)keys[i] << 32 | (unsigned)i : ~0ull;
+    __syncthreads();
+    for (int k = 2; k <= padded; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int p = t; p < padded >> 1; p += 1024) {
+                const int lo = 2 * p - (p & (j - 1)), hi = lo + j;
+                const unsigned long long x = a[lo], y = a[hi];
+                if ((x > y) == ((lo & k) == 0)) {
+                    a[lo] = y;
+                    a[hi] = x;
+                }
+            }
+            // the next stage's stride is j / 2, or k when this one ends a merge
+            if (j >= 64 || (j == 1 && k >= 64)) __syncthreads();
+            else __syncwarp();
+        }
+    __syncthreads();
+    // the payloads move through registers: they are sorted in place
+#pragma unroll
+    for (int u = 0; u < kSortSmall / 1024; u++) {
+        const int i = t + u * 1024;
+        val[u] = i < n ? vals[(unsigned)a[i]] : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kSortSmall / 1024; u++) {
+        const int i = t + u * 1024;
+        if (i < n) {
+            keys[i] = (uint32_t)(a[i] >> 32);
+            vals[i] = val[u];
+        }
+    }
+}
+
 static void rs_passes(uint32_t* k0, int* v0, uint32_t* k1, int* v1, uint32_t* hist, uint32_t* tot,
                       int n, int nblocks, int first_pass, int npasses, cudaStream_t st,
                       const Ctl* ctl, int gated) {
+    if (n <= kSortSmall && first_pass == 0 && npasses == 4) {
+        int padded = 64;
+        while (padded < n) padded *= 2;
+        if (n > 0) k_sort_small<<<1, 1024, 0, st>>>(k0, v0, n, padded, ctl, gated);
+        return;
+    }
     uint32_t* ks[2] = {k0, k1};
     int* vs[2] = {v0, v1};
     for (int p = 0; p < npasses; p++) {
