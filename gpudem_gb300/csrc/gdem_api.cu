@@ -651,10 +651,10 @@ struct Impl : EngineBase {
             double si = d.inner_skin > 0. ? d.inner_skin : 0.1 * rmax;
             if (si > skin) si = skin;
             v.inner_on = 1;
-            v.inner_skin = si;
             if (n < (1 << kHintShift)) v.row_mask = (1u << kHintShift) - 1u;
             v.inner_skinf = (float)si;
-            v.inner_thresh_sqf = (float)(0.25 * si * si);
+            v.skinf = (float)skin;
+            v.inner_adapt = d.inner_skin > 0. ? 0 : 1;
         }
         v.invdx = v.invdy = v.invdz = 1. / cell;
         v.sizex = (int)ceil((v.maxx - v.minx) / cell) + 2;
@@ -876,6 +876,7 @@ struct Impl : EngineBase {
         }
         Ctl c0;
         memset(&c0, 0, sizeof(c0));
+        c0.inner_next = v.inner_skinf;
         CKE(cudaMemcpyAsync(v.ctl, &c0, sizeof(Ctl), cudaMemcpyHostToDevice, st));
         if (v.store_forces) {
             CKE(cudaMemsetAsync(v.fx, 0, sizeof(double) * n, st));

@@ -109,7 +109,10 @@ struct Ctl {
     unsigned irefresh;        // mixed mode: the inner rows are to be rebuilt
     unsigned hold;            // chained steps: rows are to be rebuilt, or no step remains: the rest of the chain passes
     int remaining;            // chained steps still to take
+    float inner_next;         // inner skin of the next inner rows
+    float inner_thresh_sq;    // square of half the skin of the current ones
     int pad;
+    unsigned long long inner_at, inner_lists;  // steps and list rebuilds at the last inner rows
     unsigned long long inner_builds;
     unsigned wall_alloc;      // entries taken from the cell wall-candidate buffer (this rebuild)
     unsigned ncell_list;      // occupied cells listed in cell_list (this rebuild)
@@ -186,9 +189,8 @@ struct View {
     int* innw;                       // ... and the wall-row triangles within r + inner skin
     int* ninnw;
     float4* refi;
-    int inner_on;
-    double inner_skin;
-    float inner_skinf, inner_thresh_sqf;
+    int inner_on, inner_adapt;       // adapt: the skin follows how long the rows last (k_inner)
+    float inner_skinf, skinf;        // the inner skin (adapting: the least), the list skin
     // inner rows with slot hints: an entry is the partner's storage index in
     // its low kHintShift bits and, above them, 1 + the partner's history slot
     // as last seen (0: not known); row_mask keeps the index (all ones when

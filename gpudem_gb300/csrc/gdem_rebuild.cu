@@ -1079,6 +1079,7 @@ __global__ void __launch_bounds__(kBlock) k_inner(View<T> v) {
     if (ctl->irefresh == 0u) return;
     const int n = v.n;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const float skin = ctl->inner_next;
     if constexpr (T::mixed) {
         if (i < n) {
             const SBank<T> S = v.S[ctl->s];
@@ -1086,7 +1087,7 @@ __global__ void __launch_bounds__(kBlock) k_inner(View<T> v) {
             int m = 0;
             if (hi.w > 0.f) {
                 const int nn = v.nnei[i];
-                const float cut = v.inner_skinf + v.nb_delta;
+                const float cut = skin + v.nb_delta;
                 const bool hints = v.row_mask != 0xFFFFFFFFu;
                 const PBank<T> P = v.P[ctl->p];
                 // the first kInnerKeys history keys in registers for the
@@ -1134,7 +1135,7 @@ __global__ void __launch_bounds__(kBlock) k_inner(View<T> v) {
             if (hi.w > 0.f && v.ntri > 0) {
                 // FP32 closest feature with the cutoff widened by its error bound
                 const float4 lo = S.posl[i];
-                const float R = hi.w + lo.w + v.inner_skinf + v.nb_delta + v.wall_delta;
+                const float R = hi.w + lo.w + skin + v.nb_delta + v.wall_delta;
                 const int nw = v.nneiw[i];
                 for (int k = 0; k < nw; k++) {
                     const int t = v.neiw[(size_t)k * n + i];
@@ -1158,6 +1159,21 @@ __global__ void __launch_bounds__(kBlock) k_inner(View<T> v) {
         if (threadIdx.x == 0) {
             ctl->done[3] = 0;
             ctl->irefresh = 0u;
+            ctl->inner_thresh_sq = 0.25f * skin * skin;
+            // Rows that lasted under 5 steps (a list rebuild aside, which ends them
+            // early) get a wider skin the next time, rows that lasted over 10 a
+            // narrower one: a build interrupts the chain of steps (50 us on a pour of
+            // 300,000 spheres, where every third step asked for one: 71 -> 66 us a
+            // step, and 104 -> 98 once the spheres pile up); on beds the rows last
+            // hundreds of steps and the skin stays.  Results do not depend on it.
+            const unsigned long long lasted = ctl->steps - ctl->inner_at;
+            const bool own = ctl->inner_builds > 0ull && ctl->inner_lists == ctl->rebuilds;
+            ctl->inner_at = ctl->steps;
+            ctl->inner_lists = ctl->rebuilds;
+            if (v.inner_adapt && own) {
+                if (lasted < 5ull) ctl->inner_next = fminf(skin * 1.25f, v.skinf);
+                else if (lasted > 10ull) ctl->inner_next = fmaxf(skin / 1.25f, v.inner_skinf);
+            }
             ctl->inner_builds += 1ull;
         }
     }

@@ -613,7 +613,7 @@ __device__ __forceinline__ void integrate_one(const View<Mixed>& v, const SBank<
         R ex = nh.x - rf.x;
         if (per.on) ex = ex > per.half ? ex - per.Lh : (ex < -per.half ? ex + per.Lh : ex);
         const R ey = nh.y - rf.y, ez = nh.z - rf.z;
-        if (ex * ex + ey * ey + ez * ez > v.inner_thresh_sqf) votes |= kVoteInner;
+        if (ex * ex + ey * ey + ez * ez > v.ctl->inner_thresh_sq) votes |= kVoteInner;
     }
     // out of bounds (the box rounded outwards to FP32; not in a periodic x)
     R status = 1.f;

@@ -45,7 +45,7 @@ def box_limits(tris: np.ndarray, inlet_lo, inlet_hi):
 class Engine:
     """One scene on the GPU.  ``precision`` is "fp64" (bit-compatible with the
     reference CPU path) or "mixed"; ``model`` is "linear" or "hertz_mindlin".
-    ``inner_skin`` (mixed): skin of the inner rows the step scans (0: 0.1 r_max,
+    ``inner_skin`` (mixed): skin of the inner rows the step scans (0: from 0.1 r_max on,
     negative: none, the step scans the list rows); results do not depend on it."""
 
     def __init__(self, scene: Scene, precision="fp64", model="linear", reorder=True,

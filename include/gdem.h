@@ -96,8 +96,8 @@ typedef struct gdem_desc {
      * of each list row within r_i + r_j + inner_skin, rebuilt from the list rows
      * when a particle has moved half of it (and after every list rebuild).  The
      * contacts and their order are those of the list rows, so results do not
-     * change.  0: 0.1 * r_max (at most the skin); < 0: off, the step scans the
-     * list rows. */
+     * change.  0: 0.1 * r_max (at most the skin), and wider for as long as the
+     * rows last only a few steps; < 0: off, the step scans the list rows. */
     double inner_skin;
 } gdem_desc;
 

@@ -79,3 +79,21 @@ def test_graphs_follow_a_new_import_and_new_materials(precision):
         for nm in want:
             assert np.array_equal(got[nm], want[nm]), (mats, nm)
     E.close()
+
+
+def test_an_inner_skin_that_widens_changes_no_result():
+    """Fast spheres make the inner rows short-lived, so their skin grows; the
+    trajectory is that of the list rows."""
+    from gpudem_gb300 import engine
+    sc = _shower(900, 11)
+    out = []
+    for skin in (0.0, -1.0):
+        E = engine.Engine(sc, precision="mixed", model="hertz_mindlin", inner_skin=skin)
+        E.step(150)
+        out.append((E.export(history=True), E.stats()))
+        E.close()
+    (a, s), (b, t) = out
+    assert s["error_word"] == 0 and s["n_contacts"] > 0 and s["rebuilds"] == t["rebuilds"]
+    assert 0 < s["inner_builds"] < 100
+    for nm in a:
+        assert np.array_equal(a[nm], b[nm]), nm
