@@ -33,7 +33,7 @@
 //    adds its results in row order and integrates it.
 // Large scenes take a warp to a tile instead (below).  A step of a dense bed (3
 // to 5 contacts a sphere), one thread per particle and now: 100 spheres (linear
-// law) 84 and 21 us, 3,000 (Hertz-Mindlin) 668 and 30, 40,000 (linear) 1171 and
+// law) 84 and 18 us, 3,000 (Hertz-Mindlin) 668 and 30, 40,000 (linear) 1171 and
 // 140, 300,000 (Hertz-Mindlin) 5511 and 830.
 #include "gdem_step.cuh"
 
@@ -358,6 +358,167 @@ __device__ __forceinline__ void wall64(const View<FP64>& v, const SBank<FP64>& A
     S.fl[e] = (short)(kind | (slot << 2));
 }
 
+// The law of one contact by four lanes, a component to each of the first three
+// (the fourth repeats x and stores nothing): eight contacts a warp.  The vector
+// work, two thirds of a contact's FP64 instructions, is then one instruction for
+// three, and the scalars are computed by all; for tiles whose contacts would fill
+// a fraction of a warp anyway.  Operation by operation the same as pair_law64,
+// wall_law64 and finish64.
+constexpr int kSplit = 8;  // contacts a batch
+
+struct Quad {
+    int c, first;  // this lane's component; the group's first lane
+    __device__ __forceinline__ double at(double x, int k) const { return __shfl_sync(0xffffffffu, x, first + k); }
+    __device__ __forceinline__ double dot(double a, double b) const {
+        const double p = a * b, p0 = at(p, 0), p1 = at(p, 1), p2 = at(p, 2);
+        return p0 + p1 + p2;
+    }
+    __device__ __forceinline__ double cross(double a, double b) const {
+        const int u = c == 2 ? 0 : c + 1, w = c == 0 ? 2 : c - 1;
+        const double au = at(a, u), aw = at(a, w), bu = at(b, u), bw = at(b, w);
+        return au * bw - aw * bu;
+    }
+};
+__device__ __forceinline__ double comp64(const double4_32a* p, int i, int c) {
+    return reinterpret_cast<const double*>(p + i)[c];
+}
+
+// From the unit normal's component n on: overlap lap, relative velocity vr,
+// surface lever lev and relative spin rel (components), effective radius and mass
+// (Hertz-Mindlin), damping eta (linear).  `live`: the group holds a contact.
+template <int MODEL>
+__device__ __forceinline__ void law64_split(const View<FP64>& v, const Quad& G, bool live, double n, double lap, double vr,
+                                            double lev, double rel, double ri, double Rstar, double mstar, double eta,
+                                            double4_32a mi, int e, int slot, bool fresh, double* hx, double* hy,
+                                            double* hz, size_t h, Cta64& S, double* r) {
+    const int c = G.c;
+    const bool store = live && (threadIdx.x & 3) != 3;
+    const double vdn = G.dot(vr, n);
+    const double vn = vdn * n;
+    const bool pm = MODEL == 1 && v.per_particle_mat;
+    const double mu = pm ? mi.x : v.mat.mu;
+    double fn, kt, gt;
+    if (MODEL == 0) {
+        const double ki = mi.x;
+        const double del = -lap * n;
+        fn = -ki * del - eta * vn;
+        kt = ki;
+        gt = eta;
+    } else {
+        const double damp_c = pm ? mi.y : v.mat.damp_c;
+        const double sqrtRd = sqrt(Rstar * lap);
+        const double fel = v.mat.kn_c * sqrtRd * lap;
+        const double gn = damp_c * sqrt(v.mat.sn_c * sqrtRd * mstar);
+        const double fnm = fel - gn * vdn;
+        fn = fnm * n;
+        kt = v.mat.kt_c * sqrtRd;
+        gt = damp_c * sqrt(kt * mstar);
+    }
+    const double vt = (vr - vn) + G.cross(lev, n);
+    const double fnsq = G.dot(fn, fn);
+    double* const hc = c == 0 ? hx : (c == 1 ? hy : hz);
+    double d = live && slot >= 0 && !fresh ? hc[h] : 0.;
+    d = d + vt * v.dt;
+    const double ddn = G.dot(d, n);
+    d = d - ddn * n;
+    double t = -kt * d;
+    const double ftsq = G.dot(t, t);
+    if (ftsq > (mu * mu) * fnsq) {
+        if (ftsq != 0.) {
+            const double inv = 1. / (sqrt(ftsq) + 1e-15);
+            const double u = inv * t;
+            const double sc = mu * sqrt(fnsq);
+            t = sc * u;
+            const double ik = -1. / kt;
+            d = ik * t;
+        } else {
+            t = 0.;
+        }
+    } else {
+        t -= gt * vt;
+    }
+    const double tq = ri * G.cross(n, t);
+    int kind = slot < 0 ? kNormalOnly : kFull;
+    if (store) {
+        r[c * kRes64 + e] = fn;
+        if (slot >= 0) {
+            hc[h] = d;
+            r[(3 + c) * kRes64 + e] = t;
+            r[(6 + c) * kRes64 + e] = tq;
+        }
+    }
+    if (MODEL == 1 && v.mat.mu_roll > 0.) {
+        // rolling resistance, constant torque opposing the relative spin
+        const double wn = sqrt(G.dot(rel, rel));
+        if (wn > 0. && slot >= 0) {
+            const double tr = -v.mat.mu_roll * Rstar * sqrt(fnsq) / wn;
+            if (store) r[(9 + c) * kRes64 + e] = tr * rel;
+            kind = kRolling;
+        }
+    }
+    if (store && c == 0) S.fl[e] = (short)(kind | (slot << 2));
+}
+
+// Entries [e0, e0 + kSplit) of the pair list by a warp.
+template <int MODEL>
+__device__ __forceinline__ void pairs64_split(const View<FP64>& v, const SBank<FP64>& A, const PBank<FP64>& P, Cta64& S,
+                                              double* r, int base, int e0, int pairs, int lane, unsigned& err) {
+    const int n = v.n, c4 = lane & 3;
+    const Quad G = {c4 == 3 ? 0 : c4, lane & ~3};
+    const int e = min(e0 + (lane >> 2), pairs - 1);
+    const bool live = e0 + (lane >> 2) < pairs && S.es[e] != kNoHit;
+    const int a = S.eo[e], i = base + a, j = S.ej[e];
+    bool fresh;
+    const int slot = slot64(S.es, S.start[a], e, S.nc0[a], v.hist_cap, fresh);
+    const double ri = A.pos[i].w, rj = A.pos[j].w, invm = A.vel[i].w + A.vel[j].w;
+    const double wi = comp64(A.rot, i, G.c), wj = comp64(A.rot, j, G.c);
+    const double4_32a mi = P.mat[i];
+    double d = comp64(A.pos, i, G.c) - comp64(A.pos, j, G.c);
+    if (G.c == 0) d = image_dx(v, d);
+    const double dist = sqrt(G.dot(d, d));
+    const double Rs = ri + rj;
+    const double Rstar = MODEL == 1 ? ri * rj / (ri + rj) : 0., mstar = 1. / invm;
+    const double eta = MODEL == 0 ? mi.y * sqrt(mstar) : 0.;
+    const size_t h = (size_t)(slot < 0 ? 0 : slot) * n + i;
+    if (live && (lane & 3) == 0) {
+        if (slot < 0) err |= 0x4u;
+        else if (fresh) P.hid[h] = P.pid[j];
+    }
+    law64_split<MODEL>(v, G, live, d / dist, Rs - dist, comp64(A.vel, i, G.c) - comp64(A.vel, j, G.c), ri * wi + rj * wj,
+                       wi - wj, ri, Rstar, mstar, eta, mi, e, slot, fresh, P.hx, P.hy, P.hz, h, S, r);
+    if (!live && (lane & 3) == 0 && e0 + (lane >> 2) < pairs) S.fl[e] = kNone;
+}
+
+// Wall candidates [w0, w0 + kSplit) by a warp.
+template <int MODEL>
+__device__ __forceinline__ void walls64_split(const View<FP64>& v, const SBank<FP64>& A, const PBank<FP64>& P, Cta64& S,
+                                              double* r, int base, int w0, int walls, int lane, unsigned& err) {
+    const int n = v.n, c4 = lane & 3;
+    const Quad G = {c4 == 3 ? 0 : c4, lane & ~3};
+    const int w = min(w0 + (lane >> 2), walls - 1), e = kPairs64 + w;
+    const bool in = w0 + (lane >> 2) < walls, live = in && S.ws[w] != kNoHit;
+    if (!__any_sync(0xffffffffu, live)) {
+        if (in && (lane & 3) == 0) S.fl[e] = kNone;
+        return;
+    }
+    const int a = S.wo[w], i = base + a;
+    bool fresh;
+    const int slot = slot64(S.ws, S.wstart[a], w, S.ncw0[a], v.histw_cap, fresh);
+    const double rid = A.pos[i].w, invmi = A.vel[i].w, wi = comp64(A.rot, i, G.c);
+    const double4_32a mi = P.mat[i];
+    const double nrm = live ? r[G.c * kRes64 + e] : 1., lap = live ? rid - r[3 * kRes64 + e] : rid;
+    __syncwarp();
+    const double mstar = MODEL == 1 ? 1. / invmi : 0., eta = MODEL == 0 ? mi.y * mi.z : 0.;
+    const size_t h = (size_t)(slot < 0 ? 0 : slot) * n + i;
+    if (live && (lane & 3) == 0) {
+        if (slot < 0) err |= 0x8u;
+        else if (fresh) P.hwid[h] = S.wt[w];
+    }
+    law64_split<MODEL>(v, G, live, nrm, lap, comp64(A.vel, i, G.c), rid * wi, wi, rid, rid, mstar, eta, mi, e, slot, fresh,
+                       P.hwx, P.hwy, P.hwz, h, S, r);
+    if (!live && in && (lane & 3) == 0) S.fl[e] = kNone;
+}
+
 // Exclusive scan of x[0..m) into out[0..kTile] by one warp (m <= kTile <= 64).
 __device__ __forceinline__ void scan64(const int* x, int* out, int m, int lane) {
     const int a = lane < m ? x[lane] : 0, b = lane + 32 < m ? x[lane + 32] : 0;
@@ -456,7 +617,7 @@ __device__ __forceinline__ void freeze64(const View<FP64>& v, const SBank<FP64>&
 
 // One step of the m (<= kTile) particles from `base` on; false when the lists
 // are too short for them (nothing has been written then).
-template <int MODEL>
+template <int MODEL, bool SPLIT>
 __device__ __forceinline__ bool tile64(const View<FP64>& v, const SBank<FP64>& A, const SBank<FP64>& B,
                                        const PBank<FP64>& P, int base, int m, Cta64& S, double* r, bool& refresh,
                                        unsigned& err) {
@@ -606,14 +767,18 @@ __device__ __forceinline__ bool tile64(const View<FP64>& v, const SBank<FP64>& A
         }
         __syncthreads();
     }
-    // ---- contact laws, 32 entries at a time: the walls', then the pairs'
-    const int wb = any_wall ? (walls + 31) / 32 : 0, items = wb + (pairs + 31) / 32;
+    // ---- contact laws, a batch at a time: the walls', then the pairs'
+    constexpr int per_batch = SPLIT ? kSplit : 32;
+    const int wb = any_wall ? (walls + per_batch - 1) / per_batch : 0, items = wb + (pairs + per_batch - 1) / per_batch;
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(&S.item, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= items) break;
-        if (it < wb) {
+        if constexpr (SPLIT) {
+            if (it < wb) walls64_split<MODEL>(v, A, P, S, r, base, it * kSplit, walls, lane, err);
+            else pairs64_split<MODEL>(v, A, P, S, r, base, (it - wb) * kSplit, pairs, lane, err);
+        } else if (it < wb) {
             const int w = it * 32 + lane;
             if (w < walls) {
                 if (S.ws[w] != kNoHit) wall64<MODEL>(v, A, P, S, r, base, w, err);
@@ -654,7 +819,7 @@ __device__ __forceinline__ bool tile64(const View<FP64>& v, const SBank<FP64>& A
     return true;
 }
 
-template <int MODEL>
+template <int MODEL, bool SPLIT>
 __global__ void __launch_bounds__(kThreads64, 3) k_step64(View<FP64> v, cudaGraphConditionalHandle cond,
                                                               cudaGraphConditionalHandle /*inner rows: mixed mode only*/,
                                                               int use_cond) {
@@ -671,7 +836,7 @@ __global__ void __launch_bounds__(kThreads64, 3) k_step64(View<FP64> v, cudaGrap
     int part = end - first;
     for (int base = first; base < end;) {
         part = min(part, end - base);
-        if (tile64<MODEL>(v, v.S[s], v.S[s ^ 1], v.P[p], base, part, S, r, refresh, err)) {
+        if (tile64<MODEL, SPLIT>(v, v.S[s], v.S[s ^ 1], v.P[p], base, part, S, r, refresh, err)) {
             base += part;
             __syncthreads();
         } else {
@@ -1036,9 +1201,9 @@ __global__ void __launch_bounds__(32) k_step64_warp(View<FP64> v, cudaGraphCondi
     }
 }
 
-template <int MODEL>
+template <int MODEL, bool SPLIT>
 StepLaunch launch64(const View<FP64>& v, int tile) {
-    void* fn = (void*)k_step64<MODEL>;
+    void* fn = (void*)k_step64<MODEL, SPLIT>;
     static bool configured = false;
     if (!configured) {
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64<MODEL>(true));
@@ -1066,7 +1231,12 @@ StepLaunch step_launch(const View<FP64>& v, int) {
     }
     int tile = (v.n + rounds * sms - 1) / (rounds * sms);
     if (tile < 4) tile = 4;
-    return hm ? launch64<1>(v, tile) : launch64<0>(v, tile);
+    // Four particles have 20 contacts at most on beds, a batch of whole contacts
+    // for one warp and three of split ones for three.  Whole and split, a step: 100
+    // spheres (linear law) 20.9 and 18.4 us, 600 (Hertz-Mindlin) 23.0 and 20.9; 900,
+    // six to a tile, 24.4 and 24.1, and 2,000 25.0 and 31.8.
+    if (tile <= 4) return hm ? launch64<1, true>(v, tile) : launch64<0, true>(v, tile);
+    return hm ? launch64<1, false>(v, tile) : launch64<0, false>(v, tile);
 }
 
 void launch_step(const View<FP64>& v, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond) {
