@@ -603,8 +603,9 @@ void launch_step(const View<Mixed>& v, cudaStream_t st, cudaGraphConditionalHand
 // The step kernel a launch uses and its launch shape.
 // What a step kernel does beside the step (its use_cond argument): set the list
 // rebuild's condition, the inner rows' condition; belong to a chain (pass when
-// ctl->hold is set, count ctl->remaining down); end one (set the loop condition).
-constexpr int kCondLists = 1, kCondInner = 2, kChained = 4, kChainEnd = 8;
+// ctl->hold is set, count ctl->remaining down); end one (set the loop condition);
+// end its first half (the loop condition, and whether the second half runs).
+constexpr int kCondLists = 1, kCondInner = 2, kChained = 4, kChainEnd = 8, kChainMid = 16;
 // Start of `steps` chained steps; the chain's own opening (conditions of the
 // rebuilds: `any`, then `lists` and `inner` apart).
 void launch_chain_start(Ctl* ctl, int steps, cudaStream_t st);

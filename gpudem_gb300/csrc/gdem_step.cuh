@@ -24,10 +24,13 @@ inline int sm_count() {
 // pass, the rows are rebuilt, and the loop around the chain goes on with the
 // steps that remain (once more for the rows alone, when the last step asked).  `hold` is written by the last CTA of an earlier kernel
 // only, so every CTA of a kernel sees the same answer.
-__device__ __forceinline__ bool chain_passes(Ctl* ctl, int use_cond, int inner, cudaGraphConditionalHandle loop) {
+__device__ __forceinline__ bool chain_passes(Ctl* ctl, int use_cond, int inner, cudaGraphConditionalHandle loop,
+                                             cudaGraphConditionalHandle half) {
     if (!(use_cond & kChained) || ctl->hold == 0u) return false;
-    if ((use_cond & kChainEnd) && blockIdx.x == 0 && threadIdx.x == 0)
+    if ((use_cond & (kChainEnd | kChainMid)) && blockIdx.x == 0 && threadIdx.x == 0) {
         cudaGraphSetConditional(loop, ctl->remaining > 0 || ctl->refresh || (inner && ctl->irefresh) ? 1u : 0u);
+        if (use_cond & kChainMid) cudaGraphSetConditional(half, 0u);
+    }
     return true;
 }
 
@@ -45,7 +48,8 @@ __device__ __forceinline__ void step_close(Ctl* ctl, int s, int use_cond, int in
         const int left = ctl->remaining - 1;
         ctl->remaining = left;
         ctl->hold = (r | ri) != 0u || left <= 0 ? 1u : 0u;
-        if (use_cond & kChainEnd) cudaGraphSetConditional(cond, left > 0 || (r | ri) != 0u ? 1u : 0u);
+        if (use_cond & (kChainEnd | kChainMid)) cudaGraphSetConditional(cond, left > 0 || (r | ri) != 0u ? 1u : 0u);
+        if (use_cond & kChainMid) cudaGraphSetConditional(cond_inner, left > 0 && (r | ri) == 0u ? 1u : 0u);
     }
 }
 
