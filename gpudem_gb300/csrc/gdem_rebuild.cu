@@ -703,11 +703,8 @@ __global__ void __launch_bounds__(kNbBlock) k_neighbors(View<T> v, int gated) {
 template <class T, int CAP>
 static void launch_neighbors(const View<T>& v, int gated, cudaStream_t st) {
     constexpr int bytes = (3 * kNbPer * (CAP + 1) + kNbPer) * (int)sizeof(int);
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(k_neighbors<T, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        configured = true;
-    }
+    // per device; beyond the default for the widest rows only
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(k_neighbors<T, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     k_neighbors<T, CAP><<<(v.n + kNbPer - 1) / kNbPer, kNbBlock, bytes, st>>>(v, gated);
 }
 

@@ -1204,11 +1204,8 @@ __global__ void __launch_bounds__(32) k_step64_warp(View<FP64> v, cudaGraphCondi
 template <int MODEL, bool SPLIT>
 StepLaunch launch64(const View<FP64>& v, int tile) {
     void* fn = (void*)k_step64<MODEL, SPLIT>;
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64<MODEL>(true));
-        configured = true;
-    }
+    // per device, and cheap beside the graph it is built for
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem64<MODEL>(true));
     return StepLaunch{fn, dim3((v.n + tile - 1) / tile), dim3(kThreads64), smem64<MODEL>(v.mat.mu_roll > 0.)};
 }
 

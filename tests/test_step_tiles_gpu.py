@@ -86,6 +86,13 @@ def test_fp64_tiles_match_the_oracle(n, model):
 
 
 @pytest.mark.parametrize("model", ["linear", "hertz_mindlin"])
+def test_fp64_warp_tiles_match_the_oracle(model):
+    """Beyond the sizes that take a CTA to a tile."""
+    s = _same(_dense(120_001, 21, 0.05), model, (1, 2, 8))
+    assert s["n_contacts"] > 120_001 and s["n_wall_contacts"] > 0
+
+
+@pytest.mark.parametrize("model", ["linear", "hertz_mindlin"])
 def test_fp64_sphere_with_many_contacts_matches_the_oracle(model):
     s = _same(_crowded(7), model, (1, 2, 60), nei_capacity=128, hist_capacity=64, wall_capacity=64)
     assert s["n_contacts"] > 50
