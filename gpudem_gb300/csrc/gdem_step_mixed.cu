@@ -1068,14 +1068,20 @@ __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mix
 
 // The oldest B (<= 32) contacts of the ring: slots, contact law, springs, and
 // the results added to their particles' sums.
-template <int MODEL, bool PER>
+// HINTS: the row entries may carry slot hints (inner rows).  Without them every
+// contact searches its particle's keys, and key by key that is a chain of loads
+// as long as the history: so four keys at a time.  Step kernel of the 1M chute
+// bed without inner rows, key by key and four at a time: Hertz-Mindlin 704 and
+// 623 us, linear 638 and 564.  With hints the search is rare and the four keys'
+// registers cost the rest of the kernel more (416 against 420 us on that bed).
+template <int MODEL, bool PER, bool HINTS>
 __device__ __forceinline__ void coop_drain(const View<Mixed>& v, const SBank<Mixed>& A, const PBank<Mixed>& P,
                                            const CStage& S, CQueue* que, int tile, int head, int B, int lane, Force6& F,
                                            unsigned long long& touched, unsigned& err) {
     using R = float;
     const int n = v.n;
     const PerX per = per_of<PER>(v);
-    const unsigned rmask = v.row_mask;
+    const unsigned rmask = HINTS ? v.row_mask : 0xFFFFFFFFu;
     const float4* __restrict__ Aposh = A.posh;
     const float4* __restrict__ Aposl = A.posl;
     const float4* __restrict__ Avel = A.vel;
@@ -1104,11 +1110,23 @@ __device__ __forceinline__ void coop_drain(const View<Mixed>& v, const SBank<Mix
         }
         if (slot < 0) {
             renew = true;
-            for (int q = 0; q < nc0; q++)
-                if (P.hid[(size_t)q * n + iow] == j) {
-                    slot = q;
-                    break;
+            if constexpr (HINTS) {
+                // rare: a new contact, or an entry met the first time
+                for (int q = 0; q < nc0; q++)
+                    if (P.hid[(size_t)q * n + iow] == j) {
+                        slot = q;
+                        break;
+                    }
+            } else {
+                for (int q0 = 0; q0 < nc0 && slot < 0; q0 += 4) {
+                    int key[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) key[u] = q0 + u < nc0 ? P.hid[(size_t)(q0 + u) * n + iow] : -1;
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (key[u] == j) slot = q0 + u;
                 }
+            }
             if (slot >= 0) {
                 const size_t h = (size_t)slot * n + iow;
                 sp.x = P.hx[h]; sp.y = P.hy[h]; sp.z = P.hz[h];
@@ -1173,7 +1191,7 @@ __device__ __forceinline__ void coop_drain(const View<Mixed>& v, const SBank<Mix
     __syncwarp();
 }
 
-template <int MODEL, int G, int MINB, bool PER>
+template <int MODEL, int G, int MINB, bool PER, bool HINTS>
 __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<Mixed> v, cudaGraphConditionalHandle cond, cudaGraphConditionalHandle cond_inner,
                                                                     int use_cond) {
     constexpr int W = 8 * G;
@@ -1195,7 +1213,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
     const int nsub = (n + W - 1) / W;
     const int nwarps = gridDim.x * kCoopWarps;
     const int nei_rows = (n % 4 == 0) ? min(kCoopRows, v.nei_cap) : 0;
-    const unsigned rmask = v.row_mask;
+    const unsigned rmask = HINTS ? v.row_mask : 0xFFFFFFFFu;
     const PerX per = per_of<PER>(v);
     unsigned votes = 0u;
     unsigned err = 0u;
@@ -1323,7 +1341,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
                 const bool last = k0 + 4 >= most && g2 + 2 >= G;
                 while (tail - head >= 32 || (last && tail > head)) {
                     const int cnt = min(32, tail - head);
-                    coop_drain<MODEL, PER>(v, A, P, S, que, tile, head, cnt, lane, F, touched, err);
+                    coop_drain<MODEL, PER, HINTS>(v, A, P, S, que, tile, head, cnt, lane, F, touched, err);
                     head += cnt;
                 }
             }
@@ -1386,9 +1404,9 @@ void* wtma_kernel(int wall_cap) {
     }
     return fn;
 }
-template <int MODEL, int G, int MINB, bool PER>
+template <int MODEL, int G, int MINB, bool PER, bool HINTS = true>
 void* coop_kernel_of() {
-    void* fn = (void*)k_step_mixed_coop<MODEL, G, MINB, PER>;
+    void* fn = (void*)k_step_mixed_coop<MODEL, G, MINB, PER, HINTS>;
     static bool configured = false;
     if (!configured) {
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoopSmem);
@@ -1396,12 +1414,16 @@ void* coop_kernel_of() {
     }
     return fn;
 }
-// `g`: tile width over 8 (1, 2 or 4); the narrow tiles, and a periodic x,
-// exist at the default occupancy only
+// `g`: tile width over 8 (1, 2 or 4); the narrow tiles, a periodic x and the
+// search without hints exist at the default occupancy only.  Narrow tiles hold
+// scenes whose step is one tile's latency; there the two searches took the same
+// time (2,000 and 30,000 spheres), so the hinted kernels serve.
 template <int MODEL>
-void* coop_kernel(int g, int minb, bool per) {
+void* coop_kernel(int g, int minb, bool per, bool hints) {
     if (g == 1) return per ? coop_kernel_of<MODEL, 1, 5, true>() : coop_kernel_of<MODEL, 1, 5, false>();
     if (g == 2) return per ? coop_kernel_of<MODEL, 2, 5, true>() : coop_kernel_of<MODEL, 2, 5, false>();
+    if (!hints && (per || (minb != 4 && minb != 6)))
+        return per ? coop_kernel_of<MODEL, 4, 5, true, false>() : coop_kernel_of<MODEL, 4, 5, false, false>();
     if (per) return coop_kernel_of<MODEL, 4, 5, true>();
     return minb == 4 ? coop_kernel_of<MODEL, 4, 4, false>()
                      : (minb == 6 ? coop_kernel_of<MODEL, 4, 6, false>() : coop_kernel_of<MODEL, 4, 5, false>());
@@ -1440,7 +1462,8 @@ StepLaunch step_launch(const View<Mixed>& v, int reserve) {
         // 39 / 33 / 37, 50,000 42 / 40 / 38, 80,000 53 / 47 / 42.
         const int warps = 20 * sm_count();
         const int g = v.n <= 8 * warps ? 1 : (v.n <= 16 * warps ? 2 : 4);
-        void* fn = v.mat.model == 1 ? coop_kernel<1>(g, minb, per) : coop_kernel<0>(g, minb, per);
+        const bool hints = v.row_mask != 0xFFFFFFFFu;
+        void* fn = v.mat.model == 1 ? coop_kernel<1>(g, minb, per, hints) : coop_kernel<0>(g, minb, per, hints);
         const size_t smem = kCoopSmem;
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kCoopWarps * 32, smem);
