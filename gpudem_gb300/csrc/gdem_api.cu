@@ -944,11 +944,18 @@ struct Impl : EngineBase {
         }
         if (nsteps <= 0) return GDEM_OK;
         if (int rc = build_graphs()) return rc;
-        // Steps that pass still rebuild the mesh tree beside them (80 us on the
-        // 1M bed, 2 us without a tree), so with a tree the loop takes whole
-        // chains only.
+        // A few steps are faster one by one than as a chain of K whose other kernels
+        // pass (1.2 us each), though a step alone waits for a condition after its
+        // kernel, for two with inner rows.  Steps of 100 spheres in FP64 in the loop
+        // and alone (18.5 us): K = 8, two steps 23 us each, three 18.2; K = 64, eight
+        // 21.6, twelve 18.6; K = 1, two 23.9, six 19.7.  2,000 mixed, alone 18.5 to
+        // 24.6 us: K = 8, two steps 21.5, three 15.7; K = 64, two 54, six 21.5, eight
+        // 18.0.  With a tree only whole chains: steps that pass still rebuild it
+        // beside them (80 us on the 1M bed).
         const bool tree = d.bvh_every_step && mesh && mesh->ntri > 0;
-        const int looped = tree ? nsteps - nsteps % K : (nsteps > 1 ? nsteps : 0);
+        const int few = v.inner_on ? 2 + K / 12 : 2 + K / 7 + 4 / K;
+        const int alone = tree ? nsteps % K : (nsteps < few ? nsteps : 0);
+        const int looped = nsteps - alone;
         if (looped > 0) {
             launch_chain_start(v.ctl, looped, st);
             CKE(cudaGetLastError());

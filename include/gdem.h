@@ -64,7 +64,8 @@ typedef struct gdem_desc {
     int hist_wall_capacity; /* wall contacts kept in history, default 16 */
     int reorder;            /* 1: Morton-reorder particle storage at each list rebuild (default), 0: no */
     int store_forces;       /* 1: keep the last step's force and torque per particle */
-    int steps_per_graph;    /* steps unrolled per CUDA graph launch, default 8 */
+    int steps_per_graph;    /* steps taken in a chain before the device asks whether rows are to be
+                               rebuilt, default 8; results are the same for every choice */
     double dt;              /* time step (ParticleSysShared::dt) */
     double mu;              /* Coulomb friction coefficient (ParticleSysShared::mu) */
     double g[3];            /* gravity (ParticleSysShared::g) */
