@@ -501,14 +501,25 @@ struct Impl : EngineBase {
         return e;
     }
 
-    // What `launch` enqueues on the stream, captured as the nodes of `body`.
+    // What `launch` enqueues on the stream, captured as nodes of `body` after its
+    // node `dep` (if any); `last`: the node it ends with.
     template <class F>
-    cudaError_t capture_into(cudaGraph_t body, F launch) {
-        cudaError_t e = cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+    cudaError_t capture_into(cudaGraph_t body, const cudaGraphNode_t* dep, F launch, cudaGraphNode_t* last = nullptr) {
+        cudaError_t e =
+            cudaStreamBeginCaptureToGraph(st, body, dep, nullptr, dep ? 1 : 0, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) return e;
         launch();
+        if (last) {
+            cudaStreamCaptureStatus status;
+            const cudaGraphNode_t* ends = nullptr;
+            size_t cnt = 0;
+            e = cudaStreamGetCaptureInfo(st, &status, nullptr, nullptr, &ends, nullptr, &cnt);
+            if (e == cudaSuccess && cnt != 1) e = cudaErrorUnknown;
+            if (e == cudaSuccess) *last = ends[0];
+        }
         cudaGraph_t captured;
-        return cudaStreamEndCapture(st, &captured);
+        const cudaError_t e2 = cudaStreamEndCapture(st, &captured);
+        return e != cudaSuccess ? e : e2;
     }
 
     // The step kernel (and beside it the mesh tree rebuild, when asked) after
@@ -560,81 +571,100 @@ struct Impl : EngineBase {
             return rc;
         cudaGraph_t body;
         CKE(add_conditional(g, ends, nends, hl, cudaGraphCondTypeIf, &node, &body));
-        CKE(capture_into(body, [&] { launch_rebuild(v, st, /*force=*/1); }));
+        CKE(capture_into(body, nullptr, [&] { launch_rebuild(v, st, /*force=*/1); }));
         if (v.inner_on) {
             // new inner rows when some particle moved half the inner skin
             // (after a list rebuild, its own body already made them)
             const cudaGraphNode_t prev = node;
             CKE(add_conditional(g, &prev, 1, hi, cudaGraphCondTypeIf, &node, &body));
-            CKE(capture_into(body, [&] { launch_inner(v, st); }));
+            CKE(capture_into(body, nullptr, [&] { launch_inner(v, st); }));
         }
         CKE(cudaGraphInstantiate(out, g, 0));
         cudaGraphDestroy(g);
         return GDEM_OK;
     }
 
-    // Any number of steps (ctl->remaining): while steps remain, first the rows
-    // that the step before asked for, then a chain of K step kernels with no
-    // condition between them (chain_passes in gdem_step.cuh).  With condition
-    // nodes after every step a step took 10 us more than its kernel; steps of
-    // a bed before and now: 100 spheres in FP64 34 and 27 us, mixed 2,000 25
-    // and 15, 30,000 33 and 20, 250,000 102 and 89.  Chains of 16 and 32 gain
-    // under 1 us on beds and lose 5 and 14 us a step where every third step
-    // asks for new rows (a pour): each step behind it passes at 2 us.
+    // Rows asked for again within this many steps are asked for often: the steps
+    // behind each request in its chain pass, and with a mesh tree rebuild it, which
+    // then costs more than a condition after every step (8 us).  Steps of 20,000
+    // spheres over 50,000 triangles in chains and one by one, rows lasting one step:
+    // 299 and 83 us, 5 steps 111 and 85, 7 steps 77 and 77, 20 steps 81 and 77; over
+    // 300 triangles (their tree is 16 us) one step 80 and 26, and level at six.  The
+    // pour of the 1M chute (5 steps) 312 and 282.  Without a tree only rows that a
+    // fixed inner skin makes last a step or two gain (35 and 17 us), and the loop's
+    // nodes cost 2 us a request, so an adapting skin, whose rows last longer, has none.
+    int often_span() const {
+        if (d.bvh_every_step && mesh && mesh->ntri > 0) return mesh->ntri > kSortSmall ? 4 * K : K / 2 + 1;
+        return v.inner_on && !v.inner_adapt ? 1 + K / 13 : 0;
+    }
+
+    // Any number of steps (ctl->remaining): while steps remain, a chain of K step
+    // kernels with no condition between them (chain_passes in gdem_step.cuh), then
+    // the rows that one of them asked for.  With condition nodes after every step
+    // a step took 10 us more than its kernel; steps of a bed before and now: 100
+    // spheres in FP64 34 and 27 us, mixed 2,000 25 and 15, 30,000 33 and 20, 250,000
+    // 102 and 89.  Chains of 16 and 32 gain under 1 us on beds and lose 5 and 14 us
+    // a step where every third step asks for new rows (a pour): each step behind it
+    // passes at 2 us.  Where rows are asked for often (often_span), a loop within takes
+    // steps one by one with their rows behind each, until they last longer.
     int build_loop(cudaGraphExec_t* out) {
-        cudaGraph_t g, body, any, sub;
+        cudaGraph_t g, body, any, sub, often;
         CKE(cudaGraphCreate(&g, 0));
         View<T> vs = sv();
         const bool tree = d.bvh_every_step && mesh && mesh->ntri > 0;
         const StepLaunch L = step_launch(vs, tree ? kTreeReserve : 0);
         const int inner = v.inner_on;
-        cudaGraphConditionalHandle hw, ha, hl, hi = 0;
+        cudaGraphConditionalHandle hw, ha, hl, hi = 0, ho = 0, hs;
         CKE(cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
-        cudaGraphNode_t node, prev;
+        cudaGraphNode_t node, prev, ends[2];
+        int nends = 0;
         CKE(add_conditional(g, nullptr, 0, hw, cudaGraphCondTypeWhile, &node, &body));
-        CKE(cudaGraphConditionalHandleCreate(&ha, body, 0, cudaGraphCondAssignDefault));
-        CKE(capture_into(body, [&] { launch_chain_any(v.ctl, inner, ha, st); }));
-        size_t cnt = 1;
-        CKE(cudaGraphGetNodes(body, &prev, &cnt));
-        CKE(add_conditional(body, &prev, 1, ha, cudaGraphCondTypeIf, &node, &any));
-        prev = node;
-        {
-            cudaGraphNode_t q, r;
-            CKE(cudaGraphConditionalHandleCreate(&hl, any, 0, cudaGraphCondAssignDefault));
-            if (inner) CKE(cudaGraphConditionalHandleCreate(&hi, any, 0, cudaGraphCondAssignDefault));
-            CKE(capture_into(any, [&] { launch_chain_which(v.ctl, inner, hl, hi, st); }));
-            cnt = 1;
-            CKE(cudaGraphGetNodes(any, &q, &cnt));
-            CKE(add_conditional(any, &q, 1, hl, cudaGraphCondTypeIf, &r, &sub));
-            CKE(capture_into(sub, [&] { launch_rebuild(v, st, /*force=*/1); }));
-            if (inner) {
-                CKE(add_conditional(any, &r, 1, hi, cudaGraphCondTypeIf, &q, &sub));
-                CKE(capture_into(sub, [&] { launch_inner(v, st); }));
-            }
-        }
         // With a mesh tree beside each step, a step that passes still rebuilds the
-        // tree, so the second half of the chain stands in an IF of its own (a pour
-        // of the 1M chute, rows asked for every fifth step: 0.330 ms a step without,
-        // 0.322 with).
+        // tree, so the second half of the chain stands in an IF of its own (falling
+        // spheres of the 1M chute, rows asked for every 70th step: 227 us a step
+        // without, 221 with; a bed that asks for none 424.0 and 425.3).
         const int mid = tree && K > 1 ? K / 2 : K;
         cudaGraphConditionalHandle hm = hw;
         cudaGraph_t at = body;
         for (int k = 0; k < K; k++) {
-            cudaGraphNode_t ends[2];
-            int nends = 0;
-            const bool first = at != body && k == mid;
-            if (k == mid - 1 && mid < K) CKE(cudaGraphConditionalHandleCreate(&hm, body, 0, cudaGraphCondAssignDefault));
-            const int use = kChained | (k == K - 1 ? kChainEnd : 0) | (k == mid - 1 && mid < K ? kChainMid : 0);
+            const bool first = k == 0 || k == mid;
+            const int use = kChained | (k == mid - 1 && mid < K ? kChainMid : 0);
+            if (use & kChainMid) CKE(cudaGraphConditionalHandleCreate(&hm, body, 0, cudaGraphCondAssignDefault));
             if (int rc = add_step(at, first ? nullptr : &prev, vs, L, tree, hw, hm, use, ends, &nends)) return rc;
             prev = ends[0];
-            if (k == mid - 1 && mid < K) {
-                CKE(add_conditional(body, ends, nends, hm, cudaGraphCondTypeIf, &node, &sub));
-                at = sub;
+            if (use & kChainMid) {
+                CKE(add_conditional(body, ends, nends, hm, cudaGraphCondTypeIf, &node, &at));
             } else if (nends == 2) {
                 // the next step waits for both
-                CKE(cudaGraphAddEmptyNode(&node, at, ends, 2));
-                prev = node;
+                CKE(cudaGraphAddEmptyNode(&prev, at, ends, 2));
             }
+        }
+        if (mid < K) prev = node;
+        CKE(cudaGraphConditionalHandleCreate(&ha, body, 0, cudaGraphCondAssignDefault));
+        CKE(capture_into(body, &prev, [&] { launch_chain_any(v.ctl, inner, ha, hw, st); }, &prev));
+        CKE(add_conditional(body, &prev, 1, ha, cudaGraphCondTypeIf, &node, &any));
+        CKE(cudaGraphConditionalHandleCreate(&hl, any, 0, cudaGraphCondAssignDefault));
+        if (inner) CKE(cudaGraphConditionalHandleCreate(&hi, any, 0, cudaGraphCondAssignDefault));
+        const bool has_often = often_span() > 0;
+        if (has_often) CKE(cudaGraphConditionalHandleCreate(&ho, any, 0, cudaGraphCondAssignDefault));
+        CKE(capture_into(any, nullptr, [&] { launch_chain_which(v.ctl, inner, has_often, hl, hi, ho, st); }, &prev));
+        CKE(add_conditional(any, &prev, 1, hl, cudaGraphCondTypeIf, &node, &sub));
+        CKE(capture_into(sub, nullptr, [&] { launch_rebuild(v, st, /*force=*/1); }));
+        prev = node;
+        if (inner) {
+            CKE(add_conditional(any, &prev, 1, hi, cudaGraphCondTypeIf, &node, &sub));
+            CKE(capture_into(sub, nullptr, [&] { launch_inner(v, st); }));
+            prev = node;
+        }
+        if (has_often) {
+            CKE(add_conditional(any, &prev, 1, ho, cudaGraphCondTypeWhile, &node, &often));
+            CKE(capture_into(any, &node, [&] { launch_chain_again(v.ctl, hw, st); }));
+            // a step, its list rows if asked for, its inner rows (k_inner asks itself)
+            CKE(cudaGraphConditionalHandleCreate(&hs, often, 0, cudaGraphCondAssignDefault));
+            if (int rc = add_step(often, nullptr, vs, L, tree, hs, ho, kOften | kCondLists, ends, &nends)) return rc;
+            CKE(add_conditional(often, ends, nends, hs, cudaGraphCondTypeIf, &node, &sub));
+            CKE(capture_into(sub, nullptr, [&] { launch_rebuild(v, st, /*force=*/1); }));
+            if (inner) CKE(capture_into(often, &node, [&] { launch_inner(v, st); }));
         }
         CKE(cudaGraphInstantiate(out, g, 0));
         cudaGraphDestroy(g);
@@ -957,7 +987,7 @@ struct Impl : EngineBase {
         const int alone = tree ? nsteps % K : (nsteps < few ? nsteps : 0);
         const int looped = nsteps - alone;
         if (looped > 0) {
-            launch_chain_start(v.ctl, looped, st);
+            launch_chain_start(v.ctl, looped, often_span(), v.inner_on, st);
             CKE(cudaGetLastError());
             CKE(cudaGraphLaunch(gK, st));
         }

@@ -109,6 +109,8 @@ struct Ctl {
     unsigned irefresh;        // mixed mode: the inner rows are to be rebuilt
     unsigned hold;            // chained steps: rows are to be rebuilt, or no step remains: the rest of the chain passes
     int remaining;            // chained steps still to take
+    int span;                 // rows asked for within this many steps are asked for often
+    unsigned long long asked_at;  // steps when rows were last asked for
     float inner_next;         // inner skin of the next inner rows
     float inner_thresh_sq;    // square of half the skin of the current ones
     int pad;
@@ -574,6 +576,7 @@ void launch_tri_precompute(TriRec* rec, uint32_t* morton, int* idx, const double
                            const double* vy, const double* vz, const int* tv, const int* te,
                            const double* raw3, const double* dplane, int ntri, const double* gmin,
                            const double* invrange, cudaStream_t st);
+constexpr int kSortSmall = 4096;  // up to this many pairs are sorted in one launch
 void radix_sort_pairs(uint32_t* keys0, int* vals0, uint32_t* keys1, int* vals1, uint32_t* hist,
                       uint32_t* tot, int n, int nblocks, int first_pass, int npasses, cudaStream_t st);
 int rs_blocks_for(int n);
@@ -600,18 +603,22 @@ __device__ __forceinline__ void split2(double x, float& hi, float& lo) {
 // step kernels (gdem_step_fp64.cu, gdem_step_mixed.cu)
 void launch_step(const View<FP64>& v, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond);
 void launch_step(const View<Mixed>& v, cudaStream_t st, cudaGraphConditionalHandle cond, int use_cond);
-// The step kernel a launch uses and its launch shape.
 // What a step kernel does beside the step (its use_cond argument): set the list
 // rebuild's condition, the inner rows' condition; belong to a chain (pass when
-// ctl->hold is set, count ctl->remaining down); end one (set the loop condition);
-// end its first half (the loop condition, and whether the second half runs).
-constexpr int kCondLists = 1, kCondInner = 2, kChained = 4, kChainEnd = 8, kChainMid = 16;
-// Start of `steps` chained steps; the chain's own opening (conditions of the
-// rebuilds: `any`, then `lists` and `inner` apart).
-void launch_chain_start(Ctl* ctl, int steps, cudaStream_t st);
-void launch_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaStream_t st);
-void launch_chain_which(Ctl* ctl, int inner, cudaGraphConditionalHandle lists, cudaGraphConditionalHandle in,
-                        cudaStream_t st);
+// ctl->hold is set, count ctl->remaining down); end the first half of one (set
+// whether the second half runs); belong to the loop of steps that ask for rows
+// often (count down, set whether that loop goes on).
+constexpr int kCondLists = 1, kCondInner = 2, kChained = 4, kChainMid = 8, kOften = 16;
+// The kernels between chains, one thread each: the start of a call's steps; the
+// question after a chain (are any rows asked for; do steps remain); which rows,
+// and whether they are asked for often; the question after steps of their own.
+void launch_chain_start(Ctl* ctl, int steps, int span, int inner, cudaStream_t st);
+void launch_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaGraphConditionalHandle loop,
+                      cudaStream_t st);
+void launch_chain_which(Ctl* ctl, int inner, int has_often, cudaGraphConditionalHandle lists,
+                        cudaGraphConditionalHandle in, cudaGraphConditionalHandle often, cudaStream_t st);
+void launch_chain_again(Ctl* ctl, cudaGraphConditionalHandle loop, cudaStream_t st);
+// The step kernel a launch uses and its launch shape.
 struct StepLaunch {
     void* fn;
     dim3 grid, block;

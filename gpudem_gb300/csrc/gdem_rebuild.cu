@@ -178,7 +178,6 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(
 // A sort this small is bound by launches and latency: beside the step of 2,000
 // spheres the mesh tree of 300 triangles took 41 us with the eight launches of the
 // radix passes and 25 with this one, the list rebuild of 100 spheres 148 and 113.
-constexpr int kSortSmall = 4096;
 
 __global__ void __launch_bounds__(1024) k_sort_small(uint32_t* __restrict__ keys, int* __restrict__ vals, int n,
                                                      int padded, const Ctl* ctl, int gated) {
@@ -1177,24 +1176,43 @@ __global__ void __launch_bounds__(kBlock) k_inner(View<T> v) {
 }
 
 // ===================================================================== step chains
-__global__ void k_chain_start(Ctl* ctl, int steps) { ctl->remaining = steps; }
-__global__ void k_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any) {
-    cudaGraphSetConditional(any, ctl->refresh != 0u || (inner && ctl->irefresh != 0u) ? 1u : 0u);
-    ctl->hold = ctl->remaining <= 0 ? 1u : 0u;
+__global__ void k_chain_start(Ctl* ctl, int steps, int span, int inner) {
+    ctl->remaining = steps;
+    ctl->span = span;
+    ctl->hold = ctl->refresh != 0u || (inner && ctl->irefresh != 0u) ? 1u : 0u;
 }
-__global__ void k_chain_which(Ctl* ctl, int inner, cudaGraphConditionalHandle lists, cudaGraphConditionalHandle in) {
+__global__ void k_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaGraphConditionalHandle loop) {
+    ctl->hold = 0u;
+    cudaGraphSetConditional(any, ctl->refresh != 0u || (inner && ctl->irefresh != 0u) ? 1u : 0u);
+    cudaGraphSetConditional(loop, ctl->remaining > 0 ? 1u : 0u);
+}
+__global__ void k_chain_which(Ctl* ctl, int inner, int has_often, cudaGraphConditionalHandle lists,
+                              cudaGraphConditionalHandle in, cudaGraphConditionalHandle often) {
     const unsigned r = ctl->refresh;
     cudaGraphSetConditional(lists, r != 0u ? 1u : 0u);
     // a list rebuild makes new inner rows itself
     if (inner) cudaGraphSetConditional(in, r == 0u && ctl->irefresh != 0u ? 1u : 0u);
+    if (!has_often) return;
+    const unsigned long long lasted = ctl->steps - ctl->asked_at;
+    ctl->asked_at = ctl->steps;
+    cudaGraphSetConditional(often, ctl->remaining > 0 && lasted <= (unsigned long long)ctl->span ? 1u : 0u);
 }
-void launch_chain_start(Ctl* ctl, int steps, cudaStream_t st) { k_chain_start<<<1, 1, 0, st>>>(ctl, steps); }
-void launch_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaStream_t st) {
-    k_chain_any<<<1, 1, 0, st>>>(ctl, inner, any);
+__global__ void k_chain_again(Ctl* ctl, cudaGraphConditionalHandle loop) {
+    cudaGraphSetConditional(loop, ctl->remaining > 0 ? 1u : 0u);
 }
-void launch_chain_which(Ctl* ctl, int inner, cudaGraphConditionalHandle lists, cudaGraphConditionalHandle in,
-                        cudaStream_t st) {
-    k_chain_which<<<1, 1, 0, st>>>(ctl, inner, lists, in);
+void launch_chain_start(Ctl* ctl, int steps, int span, int inner, cudaStream_t st) {
+    k_chain_start<<<1, 1, 0, st>>>(ctl, steps, span, inner);
+}
+void launch_chain_any(Ctl* ctl, int inner, cudaGraphConditionalHandle any, cudaGraphConditionalHandle loop,
+                      cudaStream_t st) {
+    k_chain_any<<<1, 1, 0, st>>>(ctl, inner, any, loop);
+}
+void launch_chain_which(Ctl* ctl, int inner, int has_often, cudaGraphConditionalHandle lists,
+                        cudaGraphConditionalHandle in, cudaGraphConditionalHandle often, cudaStream_t st) {
+    k_chain_which<<<1, 1, 0, st>>>(ctl, inner, has_often, lists, in, often);
+}
+void launch_chain_again(Ctl* ctl, cudaGraphConditionalHandle loop, cudaStream_t st) {
+    k_chain_again<<<1, 1, 0, st>>>(ctl, loop);
 }
 
 static inline int grid_for(int n) { return (n + kBlock - 1) / kBlock; }

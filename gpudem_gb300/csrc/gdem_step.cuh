@@ -22,34 +22,36 @@ inline int sm_count() {
 // after another in a graph without asking the rebuild conditions in between
 // (10 us a step); when a step asks for new rows, those behind it in the chain
 // pass, the rows are rebuilt, and the loop around the chain goes on with the
-// steps that remain (once more for the rows alone, when the last step asked).  `hold` is written by the last CTA of an earlier kernel
+// steps that remain.  `hold` is written by the last CTA of an earlier kernel
 // only, so every CTA of a kernel sees the same answer.
-__device__ __forceinline__ bool chain_passes(Ctl* ctl, int use_cond, int inner, cudaGraphConditionalHandle loop,
-                                             cudaGraphConditionalHandle half) {
+__device__ __forceinline__ bool chain_passes(Ctl* ctl, int use_cond, cudaGraphConditionalHandle half) {
     if (!(use_cond & kChained) || ctl->hold == 0u) return false;
-    if ((use_cond & (kChainEnd | kChainMid)) && blockIdx.x == 0 && threadIdx.x == 0) {
-        cudaGraphSetConditional(loop, ctl->remaining > 0 || ctl->refresh || (inner && ctl->irefresh) ? 1u : 0u);
-        if (use_cond & kChainMid) cudaGraphSetConditional(half, 0u);
-    }
+    if ((use_cond & kChainMid) && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(half, 0u);
     return true;
 }
 
 // End of a step, by one thread of its last CTA: the bank flip, the step count,
 // and the graph's conditions.
 __device__ __forceinline__ void step_close(Ctl* ctl, int s, int use_cond, int inner, cudaGraphConditionalHandle cond,
-                                           cudaGraphConditionalHandle cond_inner) {
+                                           cudaGraphConditionalHandle cond2) {
+    const unsigned long long steps = ctl->steps + 1ull;
     ctl->s = s ^ 1;
-    ctl->steps += 1ull;
+    ctl->steps = steps;
     if (!use_cond) return;
     const unsigned r = atomicAdd(&ctl->refresh, 0u), ri = inner ? atomicAdd(&ctl->irefresh, 0u) : 0u;
     if (use_cond & kCondLists) cudaGraphSetConditional(cond, r ? 1u : 0u);
-    if (use_cond & kCondInner) cudaGraphSetConditional(cond_inner, ri ? 1u : 0u);
-    if (use_cond & kChained) {
+    if (use_cond & kCondInner) cudaGraphSetConditional(cond2, ri ? 1u : 0u);
+    if (use_cond & (kChained | kOften)) {
+        const bool asked = (r | ri) != 0u;
         const int left = ctl->remaining - 1;
         ctl->remaining = left;
-        ctl->hold = (r | ri) != 0u || left <= 0 ? 1u : 0u;
-        if (use_cond & (kChainEnd | kChainMid)) cudaGraphSetConditional(cond, left > 0 || (r | ri) != 0u ? 1u : 0u);
-        if (use_cond & kChainMid) cudaGraphSetConditional(cond_inner, left > 0 && (r | ri) == 0u ? 1u : 0u);
+        if (use_cond & kChained) ctl->hold = asked || left <= 0 ? 1u : 0u;
+        if (use_cond & kChainMid) cudaGraphSetConditional(cond2, asked || left <= 0 ? 0u : 1u);
+        if (use_cond & kOften) {
+            if (asked) ctl->asked_at = steps;
+            const bool often = asked || steps - ctl->asked_at < (unsigned long long)ctl->span;
+            cudaGraphSetConditional(cond2, often && left > 0 ? 1u : 0u);
+        }
     }
 }
 

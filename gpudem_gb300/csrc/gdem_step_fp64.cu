@@ -821,13 +821,13 @@ __device__ __forceinline__ bool tile64(const View<FP64>& v, const SBank<FP64>& A
 
 template <int MODEL, bool SPLIT>
 __global__ void __launch_bounds__(kThreads64, 3) k_step64(View<FP64> v, cudaGraphConditionalHandle cond,
-                                                              cudaGraphConditionalHandle half,
+                                                              cudaGraphConditionalHandle cond2,
                                                               int use_cond) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Cta64& S = *reinterpret_cast<Cta64*>(smem_raw);
     double* r = reinterpret_cast<double*>(smem_raw + sizeof(Cta64));
     Ctl* ctl = v.ctl;
-    if (chain_passes(ctl, use_cond, 0, cond, half)) return;
+    if (chain_passes(ctl, use_cond, cond2)) return;
     const int s = ctl->s, p = ctl->p;
     bool refresh = false;
     unsigned err = 0u;
@@ -848,7 +848,7 @@ __global__ void __launch_bounds__(kThreads64, 3) k_step64(View<FP64> v, cudaGrap
     if (last_block(&ctl->done[0])) {
         if (threadIdx.x == 0) {
             ctl->done[0] = 0;
-            step_close(ctl, s, use_cond, 0, cond, half);
+            step_close(ctl, s, use_cond, 0, cond, cond2);
         }
     }
 }
@@ -1182,11 +1182,11 @@ __device__ __forceinline__ void warp_tile64(const View<FP64>& v, const SBank<FP6
 // One warp per CTA: the hardware hands tiles to SMs as they come free.
 template <int MODEL>
 __global__ void __launch_bounds__(32) k_step64_warp(View<FP64> v, cudaGraphConditionalHandle cond,
-                                                    cudaGraphConditionalHandle half,
+                                                    cudaGraphConditionalHandle cond2,
                                                     int use_cond) {
     __shared__ Warp64 S;
     Ctl* ctl = v.ctl;
-    if (chain_passes(ctl, use_cond, 0, cond, half)) return;
+    if (chain_passes(ctl, use_cond, cond2)) return;
     const int s = ctl->s, p = ctl->p;
     bool refresh = false;
     unsigned err = 0u;
@@ -1196,7 +1196,7 @@ __global__ void __launch_bounds__(32) k_step64_warp(View<FP64> v, cudaGraphCondi
     if (last_block(&ctl->done[0])) {
         if (threadIdx.x == 0) {
             ctl->done[0] = 0;
-            step_close(ctl, s, use_cond, 0, cond, half);
+            step_close(ctl, s, use_cond, 0, cond, cond2);
         }
     }
 }

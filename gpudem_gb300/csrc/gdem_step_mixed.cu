@@ -723,7 +723,7 @@ template <int MODEL, int WCAP, int MINB, bool PER>
 __global__ void __launch_bounds__(kBlock, MINB) k_step_mixed(View<Mixed> v, cudaGraphConditionalHandle cond, cudaGraphConditionalHandle cond_inner,
                                                             int use_cond) {
     Ctl* ctl = v.ctl;
-    if (chain_passes(ctl, use_cond, v.inner_on, cond, cond_inner)) return;
+    if (chain_passes(ctl, use_cond, cond_inner)) return;
     const int s = ctl->s, p = ctl->p;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const SBank<Mixed> A = v.S[s];
@@ -843,7 +843,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
     WStage* stage = reinterpret_cast<WStage*>(smem_raw) + 2 * warp;
     __shared__ __align__(8) unsigned long long full[kWarps][2];
     Ctl* ctl = v.ctl;
-    if (chain_passes(ctl, use_cond, v.inner_on, cond, cond_inner)) return;
+    if (chain_passes(ctl, use_cond, cond_inner)) return;
     const int s = ctl->s, p = ctl->p;
     const SBank<Mixed> A = v.S[s];
     const SBank<Mixed> B = v.S[s ^ 1];
@@ -1201,7 +1201,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
     CQueue* que = reinterpret_cast<CQueue*>(smem_raw + 2 * kCoopWarps * sizeof(CStage)) + warp;
     __shared__ __align__(8) unsigned long long full[kCoopWarps][2];
     Ctl* ctl = v.ctl;
-    if (chain_passes(ctl, use_cond, v.inner_on, cond, cond_inner)) return;
+    if (chain_passes(ctl, use_cond, cond_inner)) return;
     const int s = ctl->s, p = ctl->p;
     const SBank<Mixed> A = v.S[s];
     const SBank<Mixed> B = v.S[s ^ 1];
