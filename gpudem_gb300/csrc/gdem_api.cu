@@ -94,6 +94,25 @@ static void host_parallel_for(int n, F f) {
     for (auto& x : th) x.join();
 }
 
+// Pages of a strided array of doubles that hold a live row's prefix, rows given
+// in ascending order.
+struct LivePages {
+    size_t row_bytes, next = 0, touched = 0;  // next: the first page not counted yet
+    int shift = 0;                            // of the page size
+    explicit LivePages(size_t stride) : row_bytes(stride * sizeof(double)) {
+        while (((size_t)1 << (shift + 1)) <= (size_t)sysconf(_SC_PAGESIZE)) shift++;
+    }
+    void add(size_t row, int live) {
+        if (live <= 0) return;
+        const size_t at = row * row_bytes, end = ((at + live * sizeof(double) - 1) >> shift) + 1;
+        const size_t first = std::max(at >> shift, next);
+        if (end > first) touched += end - first;
+        next = std::max(next, end);
+    }
+    // of n rows: are most pages live?
+    bool most(size_t n) const { return touched > 0 && 2 * (touched << shift) >= n * row_bytes; }
+};
+
 struct MeshData {
     int ntri = 0;
     char* arena = nullptr;
@@ -758,12 +777,14 @@ struct Impl : EngineBase {
             int lo = 0, rc = GDEM_OK, qmax = 0, qwmax = 0;
             double rmax = 0.;
             const char* msg = "";
+            size_t pages = 0;  // with a live particle row
         };
         std::vector<Scan> scans;
         std::mutex scan_mu;
         host_parallel_for(n, [&](int lo, int hi) {
             Scan sc;
             sc.lo = lo;
+            LivePages lp(hist ? p->hist_stride : 1);
             auto bad = [&](int rc, const char* msg) {
                 sc.rc = rc;
                 sc.msg = msg;
@@ -778,6 +799,7 @@ struct Impl : EngineBase {
                         break;
                     }
                     if (nc[i] > sc.qmax) sc.qmax = nc[i];
+                    lp.add(i, nc[i]);
                     const int* row = p->indHis + (size_t)i * p->hist_stride;
                     for (int q = 0; q < nc[i]; q++)
                         if (row[q] < 0 || row[q] >= n) {
@@ -801,16 +823,20 @@ struct Impl : EngineBase {
                         }
                 }
             }
+            sc.pages = lp.touched;
             std::lock_guard<std::mutex> lock(scan_mu);
             scans.push_back(sc);
         });
         std::sort(scans.begin(), scans.end(), [](const Scan& a, const Scan& b) { return a.lo < b.lo; });
+        LivePages live(hist ? p->hist_stride : 1);
         for (const Scan& sc : scans) {
             if (sc.rc != GDEM_OK) return failv(err, sc.rc, sc.msg);
+            live.touched += sc.pages;
             qmax = std::max(qmax, sc.qmax);
             qwmax = std::max(qwmax, sc.qwmax);
             rmax = std::max(rmax, sc.rmax);
         }
+        rows_dense = hist && live.most(n);
         // staging arrays left uninitialised: the parallel loop below writes
         // every element (first touch spread over the threads)
         HostBuf<double4_32a> pos(n);
@@ -1027,6 +1053,16 @@ struct Impl : EngineBase {
 #endif
     }
 
+    // Were most pages of the particle history rows live when they were last imported
+    // or exported?  Then an export's spring arrays are mapped while queued steps
+    // still run; else once the row lengths are known, and only if most of their
+    // pages will be written: a scene without contacts leaves the arrays, 2.4 GB at a
+    // million spheres and 100 slots, untouched (such an export 125 ms with them
+    // mapped, 54 without).  The key and wall arrays are left to the copy, whose
+    // threads share their faults (a bed of a million exported in 240 to 260 ms with all
+    // of them mapped here, in 145 to 250 with the springs alone).
+    bool rows_dense = false;
+
     // The state is gathered into pId order on the device and copied straight
     // into the caller's arrays (a million spheres: 61 ms when the arrays came
     // in storage order and the host permuted them, 4.1 ms now, of which 1 ms
@@ -1045,23 +1081,24 @@ struct Impl : EngineBase {
         launch_gather_state(v, gather, gather_i, st);
         CKE(cudaGetLastError());
         for (const Field& q : f) map_pages(q.dst, q.bytes);
-        if (p->hist_stride > 0) {
-            const size_t rows = N * p->hist_stride;
-            if (p->numCont)
-                for (void* q : {(void*)p->deltHisx, (void*)p->deltHisy, (void*)p->deltHisz}) map_pages(q, rows * D);
-        }
+        const int stv = p->hist_stride;
+        const bool refused = (p->f || p->mom) && !v.store_forces;
+        const auto map_springs = [&] {
+            for (void* q : {p->deltHisx, p->deltHisy, p->deltHisz}) map_pages(q, N * stv * D);
+        };
+        const bool ahead = !refused && stv > 0 && p->numCont && rows_dense;
+        if (ahead) map_springs();
         for (const Field& q : f)
             if (q.dst) CKE(cudaMemcpyAsync(q.dst, q.src, q.bytes, cudaMemcpyDeviceToHost, st));
         CKE(cudaStreamSynchronize(st));
         if (p->f || p->mom) {
-            if (!v.store_forces) return failv(err, GDEM_ERR_STATE, "forces not stored (store_forces=0)");
+            if (refused) return failv(err, GDEM_ERR_STATE, "forces not stored (store_forces=0)");
             launch_gather_forces(v, gather, st);
             CKE(cudaGetLastError());
             if (p->f) CKE(cudaMemcpyAsync(p->f, gather, 3 * N * D, cudaMemcpyDeviceToHost, st));
             if (p->mom) CKE(cudaMemcpyAsync(p->mom, gather + 3 * N, 3 * N * D, cudaMemcpyDeviceToHost, st));
             CKE(cudaStreamSynchronize(st));
         }
-        const int stv = p->hist_stride;
         if (stv <= 0 || !(p->numCont || p->numContWall)) return GDEM_OK;
         Ctl c;
         CKE(cudaMemcpy(&c, v.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
@@ -1074,10 +1111,17 @@ struct Impl : EngineBase {
             CKE(cudaMemcpyAsync(cnt, gather_i, N * sizeof(int), cudaMemcpyDeviceToHost, st));
             CKE(cudaStreamSynchronize(st));
             int rows = 0;
-            for (int q = 0; q < n; q++) rows = std::max(rows, std::min(cnt[q], stv));
+            LivePages lp(stv);
+            for (int q = 0; q < n; q++) {
+                const int live = std::min(cnt[q], stv);
+                rows = std::max(rows, live);
+                lp.add(q, live);
+            }
+            if (!wall) rows_dense = lp.most(N);
             if (rows == 0 || !(ind || X || Y || Z)) return GDEM_OK;
             launch_gather_history(v, wall, rows, st);
             CKE(cudaGetLastError());
+            if (!wall && rows_dense && !ahead) map_springs();
             const size_t total = N * rows;
             HostBuf<int> id(ind ? total : 0);
             HostBuf<R> hx(X ? total : 0), hy(Y ? total : 0), hz(Z ? total : 0);
