@@ -7,15 +7,13 @@
 
 namespace gdem {
 
-// SMs of the current device.
+// SMs of the current device (asked every time: an engine of another device of the
+// process has its own).
 inline int sm_count() {
-    static const int c = [] {
-        int dev = 0, cnt = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&cnt, cudaDevAttrMultiProcessorCount, dev);
-        return cnt > 0 ? cnt : 1;
-    }();
-    return c;
+    int dev = 0, cnt = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&cnt, cudaDevAttrMultiProcessorCount, dev);
+    return cnt > 0 ? cnt : 1;
 }
 
 // A chained step kernel's first question: does it pass?  Several steps run one

@@ -951,6 +951,7 @@ struct __align__(16) CQueue {
 };
 
 constexpr size_t kCoopSmem = 2 * kCoopWarps * sizeof(CStage) + kCoopWarps * sizeof(CQueue);
+static_assert(kCoopSmem <= 48 * 1024, "beyond the default limit every device would have to raise it");
 
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, unsigned bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
@@ -1396,23 +1397,13 @@ void* wtma_kernel(int wall_cap) {
     void* fn = wall_cap <= 16   ? (void*)k_step_mixed_wtma<MODEL, 16, PER>
                : wall_cap <= 32 ? (void*)k_step_mixed_wtma<MODEL, 32, PER>
                                 : (void*)k_step_mixed_wtma<MODEL, 64, PER>;
-    static bool configured[3] = {false, false, false};
-    const int slot = wall_cap <= 16 ? 0 : (wall_cap <= 32 ? 1 : 2);
-    if (!configured[slot]) {
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kWarps * kWStageBytes);
-        configured[slot] = true;
-    }
+    // per device, and cheap beside the graph it is built for
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kWarps * kWStageBytes);
     return fn;
 }
 template <int MODEL, int G, int MINB, bool PER, bool HINTS = true>
 void* coop_kernel_of() {
-    void* fn = (void*)k_step_mixed_coop<MODEL, G, MINB, PER, HINTS>;
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoopSmem);
-        configured = true;
-    }
-    return fn;
+    return (void*)k_step_mixed_coop<MODEL, G, MINB, PER, HINTS>;
 }
 // `g`: tile width over 8 (1, 2 or 4); the narrow tiles, a periodic x and the
 // search without hints exist at the default occupancy only.  Narrow tiles hold
