@@ -108,10 +108,26 @@ class Clocks:
 
 
 def sort_launches(n_keys):
-    """Kernels of one 4-pass radix sort of n_keys keys: upsweep and scatter per
-    pass, plus a digit-scan kernel per pass above 32 tiles of 2048 keys."""
+    """Kernels of one sort of n_keys keys: one up to 4,096 keys; beyond, four
+    radix passes of upsweep and scatter, plus a digit-scan kernel per pass above
+    32 tiles of 2048 keys."""
+    if n_keys <= 4096:
+        return 1
     tiles = max(1, -(-n_keys // 2048))
     return 4 * (2 if tiles <= 32 else 3)
+
+
+def step_launches(steps, ntri, tree, st0, st1, n, chain=8):
+    """Kernels of `steps` steps in one call: the step kernel (and beside it the mesh
+    tree rebuild: keys, sort, tree) of every step, the call's opening, one kernel
+    between chains, and those of each list rebuild (keys, sort, reorder and, in
+    mixed mode, its inverse order, cell clear, cell ranges, the occupied-cell list
+    (count, scan, emit), Verlet and, in FP64 mode, its FP32 positions, cell wall
+    candidates, walls) and each inner-row build.  Kernels of a chain that pass
+    because rows were asked for before them do no work and are not counted."""
+    reb = int(st1["rebuilds"] - st0["rebuilds"])
+    return (steps * (1 + (2 + sort_launches(ntri) if tree else 0)) + 1 + -(-steps // chain)
+            + reb * (11 + sort_launches(n)) + int(st1["inner_builds"] - st0["inner_builds"]))
 
 
 def algorithmic_bytes(st, n_active, s=8, s_h=8):
@@ -316,15 +332,7 @@ def run_engine(args):
                    "wall_contacts_per_sphere": round(stk["n_wall_contacts"] / max(stk["n_active"], 1), 3),
                    **extra},
         "clocks": clk.summary(),
-        # one step kernel per step (+ the mesh tree rebuild: keys, 4 sort
-        # passes, tree) + the kernels of each list rebuild (keys, 4 sort passes,
-        # reorder (+ its inverse order in mixed mode), cell clear, cell ranges,
-        # the occupied-cell list (count, scan, emit), Verlet (+ the FP32
-        # position copy in FP64 mode), cell wall candidates, walls) + each
-        # inner-row build
-        "gpu_launches": args.steps * (1 + (0 if args.bvh_once else 2 + sort_launches(int(sc.tris.shape[0]))))
-                        + reb * (11 + sort_launches(sc.n))
-                        + int(st1["inner_builds"] - st0["inner_builds"]),
+        "gpu_launches": step_launches(args.steps, int(sc.tris.shape[0]), not args.bvh_once, st0, st1, sc.n),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_source,
                      "peak_kind": f"{peak_kind} hbm_gbs",
@@ -593,8 +601,8 @@ def run_batched(args):
                       "one_by_one_value": seq_value, "one_by_one_steps_per_scene": seq_steps,
                       "batched_over_one_by_one": value / seq_value, "rebuilds_in_timed_region": reb},
            "clocks": clk.summary(),
-           "gpu_launches": args.steps + reb * (11 + sort_launches(packed.n))
-                           + int(st1["inner_builds"] - st0["inner_builds"])}
+           "gpu_launches": step_launches(args.steps, int(packed.tris.shape[0]), False, st0, st1, packed.n,
+                                         chain=kw["steps_per_graph"])}
     print(json.dumps(out))
 
 

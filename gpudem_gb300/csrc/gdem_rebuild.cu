@@ -452,8 +452,8 @@ __global__ void k_cell_ranges(View<T> v, int gated) {
 // every cell inside the grid, compacted by a count per block of kBlock
 // positions, one exclusive scan over the blocks and an emit that ranks each
 // start within its block.  Neighbouring entries are neighbouring cells, so
-// the wall-candidate traversals of neighbouring threads (k_cell_walls) walk
-// much the same part of the mesh tree.
+// the groups of lanes beside one another in k_cell_walls test much the same
+// part of the mesh tree.
 template <class T>
 __device__ __forceinline__ bool is_cell_start(const View<T>& v, int q) {
     if (q >= v.n) return false;
@@ -1057,10 +1057,11 @@ __global__ void __launch_bounds__(kBlock) k_wall_lists(View<T> v, int gated) {
 // ===================================================================== inner rows
 // Mixed mode: the partners of each list row within r_i + r_j + inner skin,
 // in row order (so in partner-pId order), the wall-row triangles within
-// r_i + inner skin (FP64 closest feature, in row order), and the high-part
-// positions they were taken at.  The test runs on the high parts with the list prefilter's
-// error bound added to the cutoff, so it keeps every pair that is within the
-// cutoff in exact arithmetic.  A pair left out is more than the inner skin
+// r_i + inner skin (in row order), and the high-part positions they were taken
+// at.  Both tests run in FP32, the pairs' on the high parts with the list
+// prefilter's error bound added to the cutoff, the walls' closest feature with
+// its own as well, so they keep all that is within the cutoff in exact
+// arithmetic.  A pair left out is more than the inner skin
 // apart, and it cannot touch before some particle has moved half the inner
 // skin, when the step asks for new rows (ctl->irefresh); every list rebuild
 // asks too.  Gated on that request in every launch mode.

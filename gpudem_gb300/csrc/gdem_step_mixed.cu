@@ -1,6 +1,6 @@
 // Mixed-precision step kernel of the GB300 DEM engine.
 //
-// Same step as the FP64 kernel (gdem_step.cuh: contacts from the Verlet and
+// Same step as the FP64 kernel (gdem_step_fp64.cu: contacts from the Verlet and
 // wall lists, tangential history, symplectic Euler, refresh test, out-of-box
 // marking), arranged so that GB300's scarce FP64 pipe is used a few times per
 // particle instead of per neighbour:
