@@ -79,6 +79,10 @@ class Clocks:
 
     def __exit__(self, *a):
         if self.p is not None:
+            # a region shorter than nvidia-smi's own start: its first sample, then
+            t0 = time.time()
+            while os.path.getsize(self.path) == 0 and self.p.poll() is None and time.time() - t0 < 2.0:
+                time.sleep(0.005)
             self.p.terminate()
             try:
                 self.p.wait(timeout=5)
