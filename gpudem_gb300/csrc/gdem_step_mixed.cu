@@ -262,6 +262,7 @@ __device__ __forceinline__ void step_epilogue(Ctl* ctl, int s, int inner, unsign
 struct Own {
     float4 wi, hi, li, vi, vl, wl, rh;
     int nn, nw, nc, ncw;
+    const float* inner_sq;  // square of half the inner skin
 };
 
 // Per-particle contact constants (Hertz-Mindlin: the scene's friction and
@@ -613,7 +614,7 @@ __device__ __forceinline__ void integrate_one(const View<Mixed>& v, const SBank<
         R ex = nh.x - rf.x;
         if (per.on) ex = ex > per.half ? ex - per.Lh : (ex < -per.half ? ex + per.Lh : ex);
         const R ey = nh.y - rf.y, ez = nh.z - rf.z;
-        if (ex * ex + ey * ey + ez * ez > v.ctl->inner_thresh_sq) votes |= kVoteInner;
+        if (ex * ex + ey * ey + ez * ez > *o.inner_sq) votes |= kVoteInner;
     }
     // out of bounds (the box rounded outwards to FP32; not in a periodic x)
     R status = 1.f;
@@ -744,6 +745,8 @@ __global__ void __launch_bounds__(kBlock, MINB) k_step_mixed(View<Mixed> v, cuda
         o.nw = __ldg(&v.nneiw[i]);
         o.nc = P.nc[i];
         o.ncw = P.ncw[i];
+        const float inner_sq = ctl->inner_thresh_sq;
+        o.inner_sq = &inner_sq;
         step_one<MODEL, WCAP, PER>(v, A, B, P, i, o, votes, err);
     }
     step_epilogue(ctl, s, v.inner_on, votes, err, cond, cond_inner, use_cond);
@@ -893,6 +896,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
             o.nw = S.nneiw[lane];
             o.nc = S.nc[lane];
             o.ncw = S.ncw[lane];
+            o.inner_sq = &ctl->inner_thresh_sq;
             step_one<MODEL, WCAP, PER>(v, A, B, P, i, o, votes, err, &S.nei[0][lane], nei_rows);
         }
         __syncwarp();
@@ -929,7 +933,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
 // share an SM with a large L1 beside them for the neighbour and history
 // gathers.
 constexpr int kCoopWarps = 4;
-constexpr int kCoopRows = 4;   // staged row entries: those of the first pass
+constexpr int kCoopRows = 4;   // staged row entries at most: those of the first pass
 
 struct __align__(16) CStage {
     float4 posh[32], posl[32], vel[32], rot[32];
@@ -948,6 +952,11 @@ struct __align__(16) CQueue {
     float f[6][32];           // force and torque of each contact of the batch being drained
     unsigned owned[32];       // the positions of a drained batch each lane owns (bit b: head + b)
     int nc[32];               // history length so far
+    // Square of half the inner skin, read from the control block once a kernel.
+    // Read for every particle it came from L2 each time (the tile counter beside it
+    // is an atomic): step kernel of a million spheres that hardly touch 62 and 53
+    // us, in a channel with one contact to five 98 and 95.
+    float inner_sq;
 };
 
 constexpr size_t kCoopSmem = 2 * kCoopWarps * sizeof(CStage) + kCoopWarps * sizeof(CQueue);
@@ -1064,7 +1073,8 @@ __device__ __forceinline__ void coop_walls(const View<Mixed>& v, const PBank<Mix
         }
         __syncwarp();
     }
-    if (active) P.ncw[i] = surviving(wtouched, ncw);
+    const int left = surviving(wtouched, ncw);
+    if (active && left != S.ncw[lane]) P.ncw[i] = left;
 }
 
 // The oldest B (<= 32) contacts of the ring: slots, contact law, springs, and
@@ -1213,12 +1223,16 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
     const int n = v.n;
     const int nsub = (n + W - 1) / W;
     const int nwarps = gridDim.x * kCoopWarps;
-    const int nei_rows = (n % 4 == 0) ? min(kCoopRows, v.nei_cap) : 0;
+    // Full tiles stage their first entries only, narrow ones, whose latency is the
+    // step, four.  Full tiles with four and one: 1M chute bed 411 and 398 us, its
+    // pour 250 and 240, lattice 53 and 52, channel 95 and 97.
+    const int nei_rows = (n % 4 == 0) ? (G == 4 ? 1 : min(kCoopRows, v.nei_cap)) : 0;
     const unsigned rmask = HINTS ? v.row_mask : 0xFFFFFFFFu;
     const PerX per = per_of<PER>(v);
     unsigned votes = 0u;
     unsigned err = 0u;
     if (lane == 0) {
+        que->inner_sq = ctl->inner_thresh_sq;
         mbar_init(&full[warp][0], 1);
         mbar_init(&full[warp][1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1269,14 +1283,10 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
         unsigned long long touched = 0ull;
         // ---- rows: lane 4 a + q tests entries q, q + 4, ... of particle
         // 8 g + a of each group g
-        int nn[G], most = 0;
+        const int own = active ? S.nnei[lane] : 0, most = __reduce_max_sync(0xffffffffu, own);
+        int nn[G];
 #pragma unroll
-        for (int g = 0; g < G; g++) {
-            const int a = 8 * g + (lane >> 2);
-            nn[g] = tile + a < n && S.rot[a].w == 1.f ? S.nnei[a] : 0;
-            most = max(most, nn[g]);
-        }
-        most = __reduce_max_sync(0xffffffffu, most);
+        for (int g = 0; g < G; g++) nn[g] = __shfl_sync(0xffffffffu, own, 8 * g + (lane >> 2));
         const float delta = v.nb_delta;
         int head = 0, tail = 0;
         // the entries of a pass are loaded during the pass before it (narrow
@@ -1320,6 +1330,11 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
                 if (c > 0 || (c < 0 && exact_contact(hi, S.posl[a], hj[g], __ldg(&Aposl[e[g] & rmask]), per)))
                     near |= 1u << g;
             }
+            // a pass that found nothing leaves the ring as it is (with the row
+            // lengths read once and the walls passed by where there are none, the
+            // kernel of the 1M chute bed 420 -> 411 us, of the channel 102 -> 98)
+            const bool none = !__any_sync(0xffffffffu, near != 0u);
+            if (none && !(k0 + 4 >= most && tail > head)) continue;
             // two groups at a time into the ring, which is then drained
 #pragma unroll 1
             for (int g2 = 0; g2 < G; g2 += 2) {
@@ -1348,10 +1363,14 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
             }
         }
         // ---- wall contacts, the geometry over the whole warp
-        coop_walls<MODEL, PER>(v, P, S, que, tile, lane, active, active ? S.nneiw[lane] : 0, S.ncw[lane], F, err);
+        const int nw = active ? S.nneiw[lane] : 0;
+        if (__any_sync(0xffffffffu, nw > 0))
+            coop_walls<MODEL, PER>(v, P, S, que, tile, lane, active, nw, S.ncw[lane], F, err);
+        else if (active && S.ncw[lane] > 0) P.ncw[i] = 0;
         if (active) {
             const Mat mt = own_material<MODEL>(v, P, i, S.posh[lane].w, S.vel[lane].w);
-            P.nc[i] = surviving(touched, que->nc[lane]);
+            const int left = surviving(touched, que->nc[lane]);
+            if (left != S.nc[lane]) P.nc[i] = left;
             Own o;
             o.wi = S.rot[lane];
             o.hi = S.posh[lane];
@@ -1360,6 +1379,7 @@ __global__ void __launch_bounds__(kCoopWarps * 32, MINB) k_step_mixed_coop(View<
             o.vl = __ldg(&A.vell[i]);
             o.wl = __ldg(&A.rotl[i]);
             o.rh = __ldg(&v.refh[i]);
+            o.inner_sq = &que->inner_sq;
             integrate_one<PER>(v, B, i, o, mt.invmoi, F, votes, err);
         }
         __syncwarp();
