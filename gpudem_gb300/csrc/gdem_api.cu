@@ -94,24 +94,21 @@ static void host_parallel_for(int n, F f) {
     for (auto& x : th) x.join();
 }
 
-// Pages of a strided array of doubles that hold a live row's prefix, rows given
-// in ascending order.
-struct LivePages {
-    size_t row_bytes, next = 0, touched = 0;  // next: the first page not counted yet
-    int shift = 0;                            // of the page size
-    explicit LivePages(size_t stride) : row_bytes(stride * sizeof(double)) {
-        while (((size_t)1 << (shift + 1)) <= (size_t)sysconf(_SC_PAGESIZE)) shift++;
-    }
-    void add(size_t row, int live) {
-        if (live <= 0) return;
-        const size_t at = row * row_bytes, end = ((at + live * sizeof(double) - 1) >> shift) + 1;
-        const size_t first = std::max(at >> shift, next);
-        if (end > first) touched += end - first;
-        next = std::max(next, end);
-    }
-    // of n rows: are most pages live?
-    bool most(size_t n) const { return touched > 0 && 2 * (touched << shift) >= n * row_bytes; }
-};
+// Does a row of most pages of a strided array of doubles hold something (rows of
+// `stride`, row q's first cnt[q])?  Rows looked at until a page's first that does.
+static bool most_pages_live(const int* cnt, size_t n, size_t stride) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE), row = stride * sizeof(double);
+    if (row > 2 * page) return false;  // what a row holds is a small part of it
+    const size_t per = std::max<size_t>(1, page / row);
+    size_t live = 0, pages = 0;
+    for (size_t lo = 0; lo < n; lo += per, pages++)
+        for (size_t q = lo; q < std::min(n, lo + per); q++)
+            if (cnt[q] > 0) {
+                live++;
+                break;
+            }
+    return live > 0 && 2 * live >= pages;
+}
 
 struct MeshData {
     int ntri = 0;
@@ -777,14 +774,12 @@ struct Impl : EngineBase {
             int lo = 0, rc = GDEM_OK, qmax = 0, qwmax = 0;
             double rmax = 0.;
             const char* msg = "";
-            size_t pages = 0;  // with a live particle row
         };
         std::vector<Scan> scans;
         std::mutex scan_mu;
         host_parallel_for(n, [&](int lo, int hi) {
             Scan sc;
             sc.lo = lo;
-            LivePages lp(hist ? p->hist_stride : 1);
             auto bad = [&](int rc, const char* msg) {
                 sc.rc = rc;
                 sc.msg = msg;
@@ -799,7 +794,6 @@ struct Impl : EngineBase {
                         break;
                     }
                     if (nc[i] > sc.qmax) sc.qmax = nc[i];
-                    lp.add(i, nc[i]);
                     const int* row = p->indHis + (size_t)i * p->hist_stride;
                     for (int q = 0; q < nc[i]; q++)
                         if (row[q] < 0 || row[q] >= n) {
@@ -823,20 +817,17 @@ struct Impl : EngineBase {
                         }
                 }
             }
-            sc.pages = lp.touched;
             std::lock_guard<std::mutex> lock(scan_mu);
             scans.push_back(sc);
         });
         std::sort(scans.begin(), scans.end(), [](const Scan& a, const Scan& b) { return a.lo < b.lo; });
-        LivePages live(hist ? p->hist_stride : 1);
         for (const Scan& sc : scans) {
             if (sc.rc != GDEM_OK) return failv(err, sc.rc, sc.msg);
-            live.touched += sc.pages;
             qmax = std::max(qmax, sc.qmax);
             qwmax = std::max(qwmax, sc.qwmax);
             rmax = std::max(rmax, sc.rmax);
         }
-        rows_dense = hist && live.most(n);
+        rows_dense = hist && most_pages_live(nc.data(), n, p->hist_stride);
         // staging arrays left uninitialised: the parallel loop below writes
         // every element (first touch spread over the threads)
         HostBuf<double4_32a> pos(n);
@@ -1111,13 +1102,8 @@ struct Impl : EngineBase {
             CKE(cudaMemcpyAsync(cnt, gather_i, N * sizeof(int), cudaMemcpyDeviceToHost, st));
             CKE(cudaStreamSynchronize(st));
             int rows = 0;
-            LivePages lp(stv);
-            for (int q = 0; q < n; q++) {
-                const int live = std::min(cnt[q], stv);
-                rows = std::max(rows, live);
-                lp.add(q, live);
-            }
-            if (!wall) rows_dense = lp.most(N);
+            for (int q = 0; q < n; q++) rows = std::max(rows, std::min(cnt[q], stv));
+            if (!wall) rows_dense = rows > 0 && most_pages_live(cnt, N, stv);
             if (rows == 0 || !(ind || X || Y || Z)) return GDEM_OK;
             launch_gather_history(v, wall, rows, st);
             CKE(cudaGetLastError());
