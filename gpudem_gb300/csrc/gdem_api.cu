@@ -711,8 +711,11 @@ struct Impl : EngineBase {
         v.skin = skin;
         // how far a cell's wall candidates reach: any particle's cutoff
         // r + skin (mixed rows also widen it by the FP32 error bounds), plus a
-        // margin far above the rounding of a position's cell coordinate
-        v.cw_reach = rmax + skin + (T::mixed ? (double)v.nb_delta + 1e-9 : 0.) + 1e-6 * cell;
+        // margin far above the rounding of a position's cell coordinate and, in
+        // FP32, of the cell's own bounds (under 5 of nb_delta's 8 ulps of a
+        // coordinate, and 1e-7 of a cell wider than the box)
+        v.cw_reach = nextafterf((float)(rmax + skin + (T::mixed ? (double)v.nb_delta + 1e-9 : 0.) + (double)v.nb_delta +
+                                        1e-6 * cell), INFINITY);
         v.thresh_sq = thresh * thresh;
         v.thresh_sqf = (float)v.thresh_sq;
         // inner rows (mixed mode): a tenth of r_max by default, never more than the skin
@@ -741,6 +744,9 @@ struct Impl : EngineBase {
         if (v.sizex > 1024 || v.sizey > 1024 || v.sizez > 1024)
             return failv(err, GDEM_ERR_RANGE, "cell grid exceeds 1024 cells per axis (10-bit Morton keys)");
         v.ncells = v.sizex * v.sizey * v.sizez;
+        v.cellw[0] = (float)(1. / v.invdx);
+        v.cellw[1] = (float)(1. / v.invdy);
+        v.cellw[2] = (float)(1. / v.invdz);
         Arena Cc;
         Cc.add(&v.cell_start, v.ncells);
         Cc.add(&v.cell_end, v.ncells);

@@ -229,7 +229,8 @@ struct View {
                                      // (the cells the wall candidates are found for)
     int* cell_bc;                    // [blocks of kBlock sorted positions + 1] cell starts per block, scanned
     int cw_cap;                      // capacity of cw_list
-    double cw_reach;                 // r_max + skin (+ the mixed rows' widening) + margin
+    float cw_reach;                  // r_max + skin (+ the mixed rows' widening) + margins
+    float cellw[3];                  // cell widths
     int seg_off[kSegMaxLevels];      // first box of each level
     int seg_top;                     // level of the root
     int ntri;

@@ -741,7 +741,11 @@ __device__ __forceinline__ bool seg_push(unsigned* stack, int& sp, int L, int k,
 // by counting.  It is bound by the latency of the box loads, one per level here;
 // a thread per cell with a stack paid it per node.  Rebuild of a bed of 30,000
 // spheres 118 -> 17 us, of 250,000 143 -> 24, of a pour of 300,000 (200,000
-// cells) 104 -> 51.
+// cells) 104 -> 51.  Beyond a million cells the chip is full and the lanes cost
+// more than they hide: a channel of ten million spheres 1,010 -> 1,710, in a
+// rebuild of 10 ms.  The cell's box is formed in FP32 with a margin for its
+// rounding; in FP64 (64 cycles a warp instruction) a rebuild of a million spheres
+// on a lattice over the chute took 997 us, now 932.
 constexpr int kCellWalls = 96;
 constexpr int kCellNodes = 128;
 constexpr int kCwLanes = 8;
@@ -755,114 +759,115 @@ __global__ void __launch_bounds__(kCwBlock) k_cell_walls(View<T> v, int gated) {
     if (gated && ctl->refresh == 0u) return;
     const int lane = threadIdx.x & 31, l = threadIdx.x % kCwLanes, group = threadIdx.x / kCwLanes;
     const unsigned gmask = ((1u << kCwLanes) - 1u) << (lane & ~(kCwLanes - 1)), below = gmask & ((1u << lane) - 1u);
-    const int c_idx = blockIdx.x * kGroups + group, cells = (int)ctl->ncell_list;
-    if (blockIdx.x * kGroups + (threadIdx.x & ~31) / kCwLanes >= cells) return;  // whole warps leave
-    const bool on = c_idx < cells;
-    const int q = v.cell_list[on ? c_idx : cells - 1];
-    if (v.ntri == 0) {
-        if (on && l == 0) v.cw_cnt[q] = 0;
-        return;
-    }
-    const uint32_t kq = v.keys[0][q];
+    const int cells = (int)ctl->ncell_list;
+    const int first = lane & ~(kCwLanes - 1);
     // the cell's grown box, one bound a lane (lanes 0..2 the lower ones, 3..5 the
-    // upper): FP64 has two lanes an SM, and eight copies of it were half the kernel
+    // upper)
     const int axis = l % 3;
     const bool upper = l >= 3;
-    const int cc = (int)compact10(axis == 0 ? kq >> 2 : (axis == 1 ? kq >> 1 : kq)) - (upper ? 0 : 1);
-    const double reach = v.cw_reach + (T::mixed ? (double)v.wall_delta : 0.);
-    const double bound = (axis == 0 ? v.minx : (axis == 1 ? v.miny : v.minz)) +
-                         (double)cc / (axis == 0 ? v.invdx : (axis == 1 ? v.invdy : v.invdz)) + (upper ? reach : -reach);
-    const int first = lane & ~(kCwLanes - 1);
-    bool past_lo = false, past_hi = false;  // periodic x: over a face
-    if (v.per_x) {
-        past_lo = (__ballot_sync(0xffffffffu, l == 0 && bound < v.minx) & gmask) != 0u;
-        past_hi = (__ballot_sync(0xffffffffu, l == 3 && bound > v.maxx) & gmask) != 0u;
-    }
-    const bool twice = past_lo || past_hi;
-    const int nimg = __any_sync(0xffffffffu, twice) ? 2 : 1;
-    // the highest level with more than kCwLanes nodes below it is the first tested
-    int top = v.seg_top;
-    while (top > 0 && ((v.ntri + (1 << (top - 1)) - 1) >> (top - 1)) <= kCwLanes) top--;
-    int* found = tris_s[group];
-    int count = 0;
-    bool full = false;
-    for (int img = 0; img < nimg; img++) {
-        const bool here = on && (img == 0 || twice);
-        // the grown box in FP32, rounded outwards
-        const double x = img == 1 && axis == 0 ? bound + (past_hi ? -v.Lx : v.Lx) : bound;
-        const float f = upper ? __double2float_ru(x) : __double2float_rd(x);
-        float flo[3], fhi[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            flo[a] = __shfl_sync(0xffffffffu, f, first + a);
-            fhi[a] = __shfl_sync(0xffffffffu, f, first + 3 + a);
+    const float w = axis == 0 ? v.cellw[0] : (axis == 1 ? v.cellw[1] : v.cellw[2]);
+    const float reach = v.cw_reach + (T::mixed ? v.wall_delta : 0.f);
+    const float edge = (axis == 0 ? v.boxf[0] : (axis == 1 ? v.boxf[1] : v.boxf[2])) + (upper ? reach : -reach);
+    // whole warps take turns: the launch has a bounded number of them
+    for (int c0 = blockIdx.x * kGroups + (threadIdx.x & ~31) / kCwLanes; c0 < cells; c0 += gridDim.x * kGroups) {
+        const int c_idx = c0 + lane / kCwLanes;
+        const bool on = c_idx < cells;
+        const int q = v.cell_list[on ? c_idx : cells - 1];
+        if (v.ntri == 0) {
+            if (on && l == 0) v.cw_cnt[q] = 0;
+            continue;
         }
-        int m = 0;  // nodes of the level above that overlap (all lanes of the group alike)
-        for (int L = top; L >= 0; L--) {
-            const int nodes = (v.ntri + (1 << L) - 1) >> L;
-            const int cands = !here || full ? 0 : (L == top ? nodes : 2 * m);
-            const int most = __reduce_max_sync(0xffffffffu, cands);
-            if (most == 0) break;  // none of the warp's cells reaches further down
-            const int* src = nodes_s[group][L & 1];
-            int* dst = L == 0 ? found : nodes_s[group][(L & 1) ^ 1];
-            int got = L == 0 ? count : 0;
-            for (int k0 = 0; k0 < most; k0 += kCwLanes) {
-                const int k = k0 + l;
-                int node = -1;
-                if (k < cands) node = L == top ? k : 2 * src[k >> 1] + (k & 1);
-                bool in = false;
-                if (node >= 0 && node < nodes) {
-                    const SegBoxF B = v.segf[v.seg_off[L] + node];
-                    in = !(B.lo[0] > fhi[0] || B.hi[0] < flo[0] || B.lo[1] > fhi[1] || B.hi[1] < flo[1] ||
-                           B.lo[2] > fhi[2] || B.hi[2] < flo[2]);
-                }
-                const unsigned hit = __ballot_sync(0xffffffffu, in) & gmask;
-                const int at = got + __popc(hit & below);
-                got += __popc(hit);
-                if (in && at < (L == 0 ? kCellWalls : kCellNodes)) dst[at] = L == 0 ? v.seg_tri[node] : node;
+        const uint32_t kq = v.keys[0][q];
+        const int cc = (int)compact10(axis == 0 ? kq >> 2 : (axis == 1 ? kq >> 1 : kq)) - (upper ? 0 : 1);
+        const float bound = fmaf((float)cc, w, edge);
+        bool past_lo = false, past_hi = false;  // periodic x: over a face
+        if (v.per_x) {
+            past_lo = (__ballot_sync(0xffffffffu, l == 0 && bound < v.perf[0]) & gmask) != 0u;
+            past_hi = (__ballot_sync(0xffffffffu, l == 3 && bound > v.perf[1]) & gmask) != 0u;
+        }
+        const bool twice = past_lo || past_hi;
+        const int nimg = __any_sync(0xffffffffu, twice) ? 2 : 1;
+        // the highest level with more than kCwLanes nodes below it is the first tested
+        int top = v.seg_top;
+        while (top > 0 && ((v.ntri + (1 << (top - 1)) - 1) >> (top - 1)) <= kCwLanes) top--;
+        int* found = tris_s[group];
+        int count = 0;
+        bool full = false;
+        for (int img = 0; img < nimg; img++) {
+            const bool here = on && (img == 0 || twice);
+            const float f = img == 1 && axis == 0 ? bound + (past_hi ? -v.Lxh : v.Lxh) : bound;
+            float flo[3], fhi[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                flo[a] = __shfl_sync(0xffffffffu, f, first + a);
+                fhi[a] = __shfl_sync(0xffffffffu, f, first + 3 + a);
             }
-            if (got > (L == 0 ? kCellWalls : kCellNodes)) full = true;
-            __syncwarp();
-            m = full ? 0 : got;
-            if (L == 0 && !full) count = got;
-        }
-    }
-    if (full) count = 0;
-    // a triangle met at both images counts once
-    int drop = 0;
-    if (nimg == 2) {
-        for (int e = l; e < count; e += kCwLanes)
-            for (int f = 0; f < e; f++)
-                if (found[f] == found[e]) {
-                    drop |= 1 << (e / kCwLanes);
-                    break;
+            int m = 0;  // nodes of the level above that overlap (all lanes of the group alike)
+            for (int L = top; L >= 0; L--) {
+                const int nodes = (v.ntri + (1 << L) - 1) >> L;
+                const int cands = !here || full ? 0 : (L == top ? nodes : 2 * m);
+                const int most = __reduce_max_sync(0xffffffffu, cands);
+                if (most == 0) break;  // none of the warp's cells reaches further down
+                const int* src = nodes_s[group][L & 1];
+                int* dst = L == 0 ? found : nodes_s[group][(L & 1) ^ 1];
+                int got = L == 0 ? count : 0;
+                for (int k0 = 0; k0 < most; k0 += kCwLanes) {
+                    const int k = k0 + l;
+                    int node = -1;
+                    if (k < cands) node = L == top ? k : 2 * src[k >> 1] + (k & 1);
+                    bool in = false;
+                    if (node >= 0 && node < nodes) {
+                        const SegBoxF B = v.segf[v.seg_off[L] + node];
+                        in = !(B.lo[0] > fhi[0] || B.hi[0] < flo[0] || B.lo[1] > fhi[1] || B.hi[1] < flo[1] ||
+                               B.lo[2] > fhi[2] || B.hi[2] < flo[2]);
+                    }
+                    const unsigned hit = __ballot_sync(0xffffffffu, in) & gmask;
+                    const int at = got + __popc(hit & below);
+                    got += __popc(hit);
+                    if (in && at < (L == 0 ? kCellWalls : kCellNodes)) dst[at] = L == 0 ? v.seg_tri[node] : node;
                 }
-        __syncwarp();
-        for (int e = l; e < count; e += kCwLanes)
-            if ((drop >> (e / kCwLanes)) & 1) found[e] = 0x7fffffff;
-        __syncwarp();
-    }
-    int kept = 0;
-    for (int e = l; e < count; e += kCwLanes) kept += found[e] != 0x7fffffff ? 1 : 0;
+                if (got > (L == 0 ? kCellWalls : kCellNodes)) full = true;
+                __syncwarp();
+                m = full ? 0 : got;
+                if (L == 0 && !full) count = got;
+            }
+        }
+        if (full) count = 0;
+        // a triangle met at both images counts once
+        int drop = 0;
+        if (nimg == 2) {
+            for (int e = l; e < count; e += kCwLanes)
+                for (int f = 0; f < e; f++)
+                    if (found[f] == found[e]) {
+                        drop |= 1 << (e / kCwLanes);
+                        break;
+                    }
+            __syncwarp();
+            for (int e = l; e < count; e += kCwLanes)
+                if ((drop >> (e / kCwLanes)) & 1) found[e] = 0x7fffffff;
+            __syncwarp();
+        }
+        int kept = 0;
+        for (int e = l; e < count; e += kCwLanes) kept += found[e] != 0x7fffffff ? 1 : 0;
 #pragma unroll
-    for (int o = kCwLanes / 2; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
-    int base = 0;
-    if (on && l == 0 && kept > 0) base = (int)atomicAdd(&ctl->wall_alloc, (unsigned)kept);
-    base = __shfl_sync(0xffffffffu, base, lane & ~(kCwLanes - 1));
-    if (base + kept > v.cw_cap) full = true;
-    if (!on) return;
-    if (l == 0) {
-        v.cw_base[q] = base;
-        v.cw_cnt[q] = full ? -1 : kept;
-    }
-    if (full) return;
-    // ascending: a triangle's place is the number of smaller ones
-    for (int e = l; e < count; e += kCwLanes) {
-        const int t = found[e];
-        if (t == 0x7fffffff) continue;
-        int place = 0;
-        for (int f = 0; f < count; f++) place += found[f] < t ? 1 : 0;
-        v.cw_list[base + place] = t;
+        for (int o = kCwLanes / 2; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
+        int base = 0;
+        if (on && l == 0 && kept > 0) base = (int)atomicAdd(&ctl->wall_alloc, (unsigned)kept);
+        base = __shfl_sync(0xffffffffu, base, lane & ~(kCwLanes - 1));
+        if (base + kept > v.cw_cap) full = true;
+        if (on && l == 0) {
+            v.cw_base[q] = base;
+            v.cw_cnt[q] = full ? -1 : kept;
+        }
+        // ascending: a triangle's place is the number of smaller ones
+        for (int e = l; on && !full && e < count; e += kCwLanes) {
+            const int t = found[e];
+            if (t == 0x7fffffff) continue;
+            int place = 0;
+            for (int f = 0; f < count; f++) place += found[f] < t ? 1 : 0;
+            v.cw_list[base + place] = t;
+        }
+        __syncwarp();  // the lists are the next cells'
     }
 }
 
@@ -1254,8 +1259,10 @@ void launch_rebuild(const View<T>& v, cudaStream_t st, int force) {
         launch_neighbors<T, 64>(v, gated, st);
     else
         launch_neighbors<T, 128>(v, gated, st);
-    // a group of lanes per occupied cell, of which there are n at most
-    k_cell_walls<T><<<(n + kCwBlock / kCwLanes - 1) / (kCwBlock / kCwLanes), kCwBlock, 0, st>>>(v, gated);
+    // a group of lanes per occupied cell, of which there are n at most; a bounded
+    // number of CTAs, since most of one per 16 particles would find no cell left
+    const int gw = (n + kCwBlock / kCwLanes - 1) / (kCwBlock / kCwLanes);
+    k_cell_walls<T><<<gw < 4096 ? gw : 4096, kCwBlock, 0, st>>>(v, gated);
     if (v.wall_cap <= 16)
         k_wall_lists<T, 16><<<g, kBlock, 0, st>>>(v, gated);
     else if (v.wall_cap <= 32)
