@@ -41,11 +41,11 @@ METRIC = "particle-steps/s at 1M spheres, FP32-mixed vs FP64 plain on 1 GB300 (e
 # poured chute bed, from a one-pass ncu capture of the DRAM byte counters on
 # that launch itself (profiles/k_step_mixed_coop_poured_bed_1M_dram.txt);
 # scaled by the spheres of a launch
-TRAFFIC_POURED_BED_PER_SPHERE = 758_400_000.0 / 999_999
+TRAFFIC_POURED_BED_PER_SPHERE = 746_871_040.0 / 999_999
 # bytes per sphere of one step-kernel launch on the periodic channel, from an
 # ncu capture of the 1M-sphere channel (the 10M one is too large to capture);
 # the launch's traffic scales with the spheres it steps
-TRAFFIC_CHANNEL_PER_SPHERE = 218_407_936.0 / 1_000_000
+TRAFFIC_CHANNEL_PER_SPHERE = 214_220_800.0 / 1_000_000
 UNIT = "particle-steps/s"
 METRIC_CHANNEL = "particle-steps/s at 10M spheres in a channel periodic in x, FP32-mixed on 1 GB300"
 
