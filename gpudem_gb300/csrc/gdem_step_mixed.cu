@@ -927,10 +927,10 @@ __global__ void __launch_bounds__(kBlock, 2) k_step_mixed_wtma(View<Mixed> v, cu
 // The kernel is bound by the latency of its gathers.  The form before tested a
 // row per lane and found the slots contact by contact, two dependent loads
 // each, in tiles of 32 only; its step kernel and this one: 2,000 spheres 23.8
-// and 15.0 us, 30,000 31.7 and 22.0, 96,000 in 48 boxes 50 and 34, 250,000
-// (linear law) 101 and 89, 1,000,000 325 and 312.  Shared memory per warp is kept small
-// (two stage buffers and the ring, 7.8 KB) so that five CTAs of four warps
-// share an SM with a large L1 beside them for the neighbour and history
+// and 15.0 us, 30,000 31.7 and 21.0, 96,000 in 48 boxes 50 and 32, 250,000
+// (linear law) 101 and 82, 1,000,000 325 and 294.  Shared memory per warp is
+// kept small (two stage buffers and the ring, 7.8 KB) so that five CTAs of four
+// warps share an SM with a large L1 beside them for the neighbour and history
 // gathers.
 constexpr int kCoopWarps = 4;
 constexpr int kCoopRows = 4;   // staged row entries at most: those of the first pass
